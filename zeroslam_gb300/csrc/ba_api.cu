@@ -30,7 +30,13 @@ using namespace zs;
 
 namespace {
 
-constexpr int kSegment = 512;  // triples per Schur segment (a warp's share)
+// Triples per Schur segment (a warp's share): 512, or in FP64 fewer where the
+// problem has too few of them to give every SM quarter four warps (152 x 4 x
+// 4), but at least four rounds of the warp's eight triples. The mixed form
+// keeps 512: its FP32 sums depend on the split.
+constexpr int64_t kSegment = 512;
+constexpr int64_t kSegmentMin = 32;
+constexpr int64_t kSchurWarps = 152 * 16;
 
 
 struct CudaError {
@@ -860,14 +866,16 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
     std::vector<int64_t> seg_ptr{0}, pair_seg_ptr{0};
     pair_i.reserve(npairs);
     pair_j.reserve(npairs);
+    const int64_t seg_len =
+        h->tsize == 4 ? kSegment : std::clamp((ntriples / kSchurWarps + 7) / 8 * 8, kSegmentMin, kSegment);
     for (int w = 0; w < nwin; ++w) {
         const int64_t kw = wp[w + 1] - wp[w];
         for (int64_t k = key_base[w]; k < key_base[w + 1]; ++k) {
             if (!pair_count[k]) continue;
             pair_i.push_back((int32_t)(wp[w] + (k - key_base[w]) / kw));
             pair_j.push_back((int32_t)(wp[w] + (k - key_base[w]) % kw));
-            for (int64_t t = pair_off[k]; t < pair_off[k + 1]; t += kSegment) {
-                seg_ptr.push_back(std::min<int64_t>(t + kSegment, pair_off[k + 1]));
+            for (int64_t t = pair_off[k]; t < pair_off[k + 1]; t += seg_len) {
+                seg_ptr.push_back(std::min<int64_t>(t + seg_len, pair_off[k + 1]));
                 seg_pair.push_back((int32_t)pair_i.size() - 1);
             }
             pair_seg_ptr.push_back((int64_t)seg_pair.size());

@@ -674,49 +674,36 @@ __device__ __forceinline__ void load_rec(const float* p, float v[20]) {
         v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
     }
 }
-__device__ __forceinline__ void load_rec(const double* p, double v[20]) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        const double2 t = __ldg(q + i);
-        v[2 * i] = t.x; v[2 * i + 1] = t.y;
-    }
-}
-
 // Partial 6 x 6 sums W_i H_j^T over one segment (<= 512 consecutive triples
-// of one pose pair), a warp per segment: lane t takes the segment's triples
-// t, t + 32, ... (consecutive lanes read consecutive pose-major records,
-// coalesced) and accumulates in T (at most 16 triples per lane); the 32 lane
-// partials meet in a fixed tree (FP32: an xor-shuffle butterfly, identical in
-// every lane; FP64: a transpose through shared memory and a column sum in
-// lane order) and the segment sum is stored in FP64. (The mixed form's S is
-// the preconditioner of its conjugate-gradient solve, launch_pcg, so FP32
-// sums suffice there.) With windows, segments of stopped windows (ctl) are
+// of one pose pair), a warp per segment, FP32 (the mixed form's S is the
+// preconditioner of its conjugate-gradient solve, launch_pcg): lane t takes
+// the segment's triples t, t + 32, ... (consecutive lanes read consecutive
+// pose-major records, coalesced), at most 16 per lane; the 32 lane partials
+// meet in an xor-shuffle butterfly, identical in every lane, and the segment
+// sum is stored in FP64. With windows, segments of stopped windows (ctl) are
 // skipped.
-template <typename T>
-constexpr int schur_seg_threads() {
-    return sizeof(T) == 8 ? 128 : 256;  // FP64: 4 warps keep the transpose buffer under 48 KB
+constexpr int kSchurThreadsF32 = 256;
+constexpr int kSchurThreadsF64 = 128;
+
+__device__ __forceinline__ bool schur_segment_active(const DevProblem& P, int64_t g, const WinCtl* __restrict__ ctl) {
+    return !(ctl && P.pose_win && !ctl[P.pose_win[P.pair_i[P.seg_pair[g]]]].active);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(schur_seg_threads<T>()) k_schur_segments(DevProblem P, const T* __restrict__ W,
-                                                                          const T* __restrict__ hpl,
-                                                                          double* __restrict__ part,
-                                                                          const WinCtl* __restrict__ ctl) {
-    constexpr int RS = RecStride<T>::value;
-    constexpr int NW = schur_seg_threads<T>() / 32;
-    __shared__ double red[sizeof(T) == 8 ? NW : 1][32][37];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kSchurThreadsF32) k_schur_segments(DevProblem P, const float* __restrict__ W,
+                                                                     const float* __restrict__ hpl,
+                                                                     double* __restrict__ part,
+                                                                     const WinCtl* __restrict__ ctl) {
+    constexpr int RS = RecStride<float>::value;
+    const int lane = threadIdx.x & 31;
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (g >= P.nsegs) return;
-    if (ctl && P.pose_win && !ctl[P.pose_win[P.pair_i[P.seg_pair[g]]]].active) return;
-    T acc[36];
+    if (g >= P.nsegs || !schur_segment_active(P, g, ctl)) return;
+    float acc[36];
 #pragma unroll
-    for (int e = 0; e < 36; ++e) acc[e] = T(0);
+    for (int e = 0; e < 36; ++e) acc[e] = 0.f;
     const int64_t t1 = P.seg_ptr[g + 1];
     for (int64_t t = P.seg_ptr[g] + lane; t < t1; t += 32) {
         const int2 tr = P.triples[t];
-        T wv[20], hv[20];
+        float wv[20], hv[20];
         load_rec(W + (int64_t)tr.x * RS, wv);
         load_rec(hpl + (int64_t)tr.y * RS, hv);
 #pragma unroll
@@ -726,28 +713,67 @@ __global__ void __launch_bounds__(schur_seg_threads<T>()) k_schur_segments(DevPr
                 acc[a * 6 + d] += wv[a * 3] * hv[d * 3] + wv[a * 3 + 1] * hv[d * 3 + 1] + wv[a * 3 + 2] * hv[d * 3 + 2];
     }
     double* out = part + g * 36;
-    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int e = 0; e < 36; ++e) {
-            T v = acc[e];
+    for (int e = 0; e < 36; ++e) {
+        float v = acc[e];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (e == lane || e == 32 + lane) out[e] = (double)v;
-        }
-    } else {
-        double (*r)[37] = red[wib];
-#pragma unroll
-        for (int e = 0; e < 36; ++e) r[lane][e] = (double)acc[e];
-        __syncwarp();
-        double v0 = 0.0;
-        for (int k = 0; k < 32; ++k) v0 += r[k][lane];
-        out[lane] = v0;
-        if (lane < 4) {
-            double v1 = 0.0;
-            for (int k = 0; k < 32; ++k) v1 += r[k][32 + lane];
-            out[32 + lane] = v1;
-        }
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        if (e == lane || e == 32 + lane) out[e] = (double)v;
     }
+}
+
+// The same sums in FP64. The FP64 pipe bounds them (one lane's multiply-add
+// per two cycles and SM quarter: a warp's instruction holds it for 64
+// cycles, whether its lanes are in use or not), so lanes must not idle: four
+// lanes share a triple, each the 3 x 3 quarter of its 6 x 6 product, and the
+// warp takes eight triples at a time. A segment of m triples then costs
+// 27 ceil(m / 8) multiply-adds per warp and 27 for the butterfly over the
+// eight groups; with a lane per triple it was 108 ceil(m / 32) and 64.
+__global__ void __launch_bounds__(kSchurThreadsF64) k_schur_segments_f64(DevProblem P, const double* __restrict__ W,
+                                                                         const double* __restrict__ hpl,
+                                                                         double* __restrict__ part,
+                                                                         const WinCtl* __restrict__ ctl) {
+    constexpr int RS = RecStride<double>::value;
+    const int lane = threadIdx.x & 31;
+    const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (g >= P.nsegs || !schur_segment_active(P, g, ctl)) return;
+    const int r3 = 3 * ((lane >> 1) & 1), c3 = 3 * (lane & 1);  // the quarter's first row and column
+    double acc[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[a][d] = 0.0;
+    const int64_t t1 = P.seg_ptr[g + 1];
+    int64_t t = P.seg_ptr[g] + (lane >> 2);
+    int2 tr = t < t1 ? P.triples[t] : make_int2(0, 0);
+    while (t < t1) {
+        const double* wp = W + (int64_t)tr.x * RS + 3 * r3;
+        const double* hp = hpl + (int64_t)tr.y * RS + 3 * c3;
+        t += 8;
+        if (t < t1) tr = P.triples[t];
+        double w[9], h[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            w[i] = __ldg(wp + i);
+            h[i] = __ldg(hp + i);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                acc[a][d] = fma(w[3 * a], h[3 * d], fma(w[3 * a + 1], h[3 * d + 1], fma(w[3 * a + 2], h[3 * d + 2], acc[a][d])));
+    }
+    double* out = part + g * 36;
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            double v = acc[a][d];
+#pragma unroll
+            for (int off = 4; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane < 4) out[(r3 + a) * 6 + c3 + d] = v;
+        }
 }
 
 // S_ij -= the pair's segment sums, added in FP64 in segment order: diagonal
@@ -1123,9 +1149,12 @@ void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStr
 template <typename T>
 void launch_schur_pairs(const DevProblem& P, DevWork& W, const WinCtl* ctl, cudaStream_t s) {
     if (P.npairs > 0) {
-        constexpr int nt = schur_seg_threads<T>();
-        const int64_t blocks = (P.nsegs * 32 + nt - 1) / nt;
-        k_schur_segments<T><<<(int)blocks, nt, 0, s>>>(P, (const T*)W.W, (const T*)W.hpl, W.partial, ctl);
+        if constexpr (sizeof(T) == 8)
+            k_schur_segments_f64<<<grid_for(32 * P.nsegs, kSchurThreadsF64), kSchurThreadsF64, 0, s>>>(
+                P, (const double*)W.W, (const double*)W.hpl, W.partial, ctl);
+        else
+            k_schur_segments<<<grid_for(32 * P.nsegs, kSchurThreadsF32), kSchurThreadsF32, 0, s>>>(
+                P, (const float*)W.W, (const float*)W.hpl, W.partial, ctl);
         note_launch();
         k_schur_assemble<<<grid_for((int64_t)P.npairs * 36), kThreads, 0, s>>>(P, W.partial, W.S, ctl);
         note_launch();
