@@ -429,7 +429,7 @@ int zs_ba_cull(zs_ba_handle* h, const int32_t* landmark_id, const int32_t* pose_
  * above the diagonal) and x may be NULL. precision: ZS_PRECISION_FP64, or
  * ZS_PRECISION_MIXED (the mixed solve's preconditioner: FP32 factor and its
  * inverse, then FP64 refinement of x).
- * Returns ZS_OK, ZS_ERR_CHOLESKY, ZS_ERR_TIMEOUT (mixed: a bounded wait between
+ * Returns ZS_OK, ZS_ERR_CHOLESKY, ZS_ERR_TIMEOUT (a bounded wait between
  * the factor's tile tasks ran out; nothing hangs) or a CUDA status. */
 int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* L, double* x, int precision);
 
@@ -442,7 +442,7 @@ int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* L, 
  * application whose device memory belongs to another allocator. This entry
  * point has no counterpart in the reference; it calls no cudaMalloc, cudaFree
  * or other allocating routine. Its device workspace is one fixed array of
- * about 2.5 MB inside this library (sized for n <= ZS_NOALLOC_MAX_N) that
+ * about 3.2 MB inside this library (sized for n <= ZS_NOALLOC_MAX_N) that
  * every device loading the library keeps until the process exits; larger n
  * returns ZS_ERR_INVALID. A, b, L and x are host pointers as in
  * zs_dense_cholesky_solve; L and x may be NULL. Runs on the current device's
@@ -453,8 +453,8 @@ int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* L, 
  * not be called on that device again. All calls share the one workspace:
  * calls that overlap on the GPU (other host threads, other streams) race.
  * Returns ZS_OK, ZS_ERR_CHOLESKY (a pivot or solve test failed),
- * ZS_ERR_INVALID (null A or b, n <= 0 or n > ZS_NOALLOC_MAX_N) or
- * ZS_ERR_CUDA / ZS_ERR_OUT_OF_MEMORY (a CUDA call failed; zs_last_error()
+ * ZS_ERR_INVALID (null A or b, n <= 0 or n > ZS_NOALLOC_MAX_N),
+ * ZS_ERR_TIMEOUT (a bounded device wait ran out) or ZS_ERR_CUDA / ZS_ERR_OUT_OF_MEMORY (a CUDA call failed; zs_last_error()
  * names it). */
 int zs_dense_cholesky_solve_noalloc(const double* A, int n, const double* b, double* L, double* x);
 

@@ -1002,6 +1002,8 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
             W.dag_flags = dalloc<int>((size_t)dag_flag_ints(n), own);
             W.dag_epoch = 0;
             ZS_CUDA(cudaMemsetAsync(W.dag_flags, 0, sizeof(int) * (size_t)dag_flag_ints(n), s));
+        } else {
+            W.fx = dalloc<char>(chol_fx_bytes(n), own);
         }
     }
     W.delta = dalloc<double>((size_t)n + 3 * (size_t)L, own);
@@ -1140,7 +1142,7 @@ void system_solve(zs_ba_handle* h) {
             ZS_CUDA(launch_preconditioner(P.n, W.S, (float*)W.F, (float*)W.X, (float*)W.XT, W.tc_scratch,
                                           W.tc_streams, h->st, kPreconditionerShift, W.dag_flags, &W.dag_epoch, s));
         else
-            ZS_CUDA((launch_factor<double, T>(P.n, W.S, (T*)W.F, (T*)W.D, h->st, s)));
+            ZS_CUDA(launch_factor(P.n, W.S, (double*)W.F, (double*)W.D, W.fx, h->st, s));
     }
     {
         PhaseScope ps(h->timer, ZS_PHASE_TRISOLVE, s);
@@ -1714,10 +1716,10 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
         ZS_CUDA(cudaMemcpyAsync(h->st, &init, sizeof(LmState), cudaMemcpyHostToDevice, s));
         launch_invert_w<double>(P, W, h->st, s);
         launch_schur<double>(P, W, h->st, s);
-        ZS_CUDA((launch_factor<double, double>(n, W.S, (double*)W.F, (double*)W.D, h->st, s)));
+        ZS_CUDA(launch_factor(n, W.S, (double*)W.F, (double*)W.D, W.fx, h->st, s));
         read_state(h);
         if (!h->st_host->solve_ok) {
-            status = ZS_ERR_CHOLESKY;
+            status = h->st_host->timeout ? ZS_ERR_TIMEOUT : ZS_ERR_CHOLESKY;
         } else {
             std::vector<double> red(kReduceBlocks * 4);
             auto dot = [&](const double* x, const double* y) {
@@ -1866,7 +1868,8 @@ int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* Lou
         if (precision == ZS_PRECISION_FP64) {
             double* dF = dalloc<double>(nn, owned);
             double* dD = dalloc<double>(1024 * (size_t)((n + 31) / 32), owned);
-            ZS_CUDA((launch_reduced_solve<double, double>(n, dA, dF, dD, db, dx, dwork, st, 0, 0.0, s)));
+            void* dfx = dalloc<char>(chol_fx_bytes(n), owned);
+            ZS_CUDA(launch_reduced_solve(n, dA, dF, dD, dfx, db, dx, dwork, st, s));
             if (Lout) {
                 Lh.resize(nn);
                 ZS_CUDA(cudaMemcpyAsync(Lh.data(), dF, nn * sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -1,12 +1,7 @@
 // Dense reduced-camera-system solve S x = b_s on the device (sm_103a).
 //
-// Factorisation: one cooperative persistent kernel over every SM performs a
-// blocked right-looking Cholesky S = L L^T on the row-major lower triangle,
-// 32-wide panels, two grid barriers per panel:
-//   phase B  L_ik = A_ik D_k^T for the rows below the panel (D_k = L_kk^-1),
-//   phase C  A_ij -= L_ik L_jk^T over the trailing lower 32 x 32 tiles; the
-//            CTA that updates the next diagonal tile first factors it and
-//            inverts its factor (look-ahead), so the next panel can start.
+// Factorisation: ba_chol_fx.cu (k_chol_fx), which also inverts L's 32 x 32
+// diagonal blocks (D_k = L_kk^-1).
 // Triangular solves: one thread-block cluster (16 CTAs, or 8 where 16 is not
 // allowed) walks the 32-row blocks with cluster barriers, each block step a
 // small GEMV with D_k; the mixed form's FP64 refinement sweeps
@@ -58,213 +53,6 @@ template <typename TS, typename TF>
 __global__ void __launch_bounds__(kThreads) k_convert(int64_t N, const TS* __restrict__ src, TF* __restrict__ dst) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < N) dst[i] = (TF)src[i];
-}
-
-// The CTA factors the b x b diagonal block at j0 (b <= 32) in shared memory,
-// right-looking, two barriers per column; pivots go to dg[] and the
-// multipliers are formed with one reciprocal per column. Writes L_jj (zero
-// above the diagonal) into F. Returns false, uniformly across the CTA, when a
-// pivot fails zeroslam's test (the block is then left unwritten).
-template <typename T>
-__device__ bool factor_diag(int n, T* F, int j0, double eps, T (*a)[kNB + 1], T* dg) {
-    const int b = min(kNB, n - j0);
-    T v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        const int i = e >> 5, m = e & 31;
-        v[q] = (i < b && m < b) ? ldg2(F + (int64_t)(j0 + i) * n + j0 + m) : (i == m ? T(1) : T(0));
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        a[e >> 5][e & 31] = v[q];
-    }
-    __syncthreads();
-    bool ok = true;
-    for (int k = 0; k < b; ++k) {
-        const T akk = a[k][k];
-        if (!((double)akk > eps)) {
-            ok = false;
-            break;
-        }
-        const T piv = sqrt(akk);
-        const T inv = T(1) / piv;
-        if (threadIdx.x > k && threadIdx.x < b) a[threadIdx.x][k] *= inv;
-        if (threadIdx.x == 0) dg[k] = piv;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = threadIdx.x + q * kThreads;
-            const int i = e >> 5, m = e & 31;
-            if (m > k && m <= i && i < b) a[i][m] -= a[i][k] * a[m][k];
-        }
-        __syncthreads();
-    }
-    if (!ok) return false;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        const int i = e >> 5, m = e & 31;
-        if (i < b && m < b) F[(int64_t)(j0 + i) * n + j0 + m] = (m < i) ? a[i][m] : (m == i ? dg[i] : T(0));
-    }
-    __syncthreads();
-    return true;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) k_chol_coop(int n, T* F, LmState* st) {
-    cg::grid_group grid = cg::this_grid();
-    __shared__ T sa[kNB][kNB + 1];
-    __shared__ T sb[kNB][kNB + 1];
-    __shared__ T dg[kNB];
-    const int nblk = (n + kNB - 1) / kNB;
-    if (ldg2(&st->skip_factor)) return;  // written by an earlier launch: uniform
-    const double eps = ldg2(&st->eps_factor);
-    const int G = gridDim.x;
-    if (blockIdx.x == 0) {
-        if (!factor_diag<T>(n, F, 0, eps, sa, dg) && threadIdx.x == 0) st->solve_ok = 0;
-    }
-    grid.sync();
-    for (int k = 0; k < nblk; ++k) {
-        if (!ld_ok(st)) return;  // read after a grid barrier: every CTA sees the same value
-        const int k0 = k * kNB;
-        const int kb = min(kNB, n - k0);
-        const int r0 = k0 + kb;
-        if (r0 >= n) break;
-        // Phase B: rows below the panel solve x L_kk^T = a by substitution
-        // (a thread per row) against L_kk in shared memory.
-        {
-            T v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = threadIdx.x + q * kThreads;
-                const int i = e >> 5, m = e & 31;
-                v[q] = (i < kb && m < kb) ? ldg2(F + (int64_t)(k0 + i) * n + k0 + m) : T(0);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = threadIdx.x + q * kThreads;
-                sb[e >> 5][e & 31] = v[q];
-            }
-            __syncthreads();
-            if (threadIdx.x < kNB) dg[threadIdx.x] = threadIdx.x < kb ? T(1) / sb[threadIdx.x][threadIdx.x] : T(0);
-            __syncthreads();
-            const int rows = n - r0;
-            const int per = (rows + G - 1) / G;
-            const int rbeg = r0 + blockIdx.x * per, rend = min(n, rbeg + per);
-            for (int row = rbeg + threadIdx.x; row < rend; row += blockDim.x) {
-                T x[kNB];
-                T* rp = F + (int64_t)row * n + k0;
-#pragma unroll
-                for (int c = 0; c < kNB; ++c) x[c] = (c < kb) ? ldg2(rp + c) : T(0);
-#pragma unroll
-                for (int c = 0; c < kNB; ++c) {
-                    T acc = x[c];
-#pragma unroll
-                    for (int m = 0; m < c; ++m) acc -= x[m] * sb[c][m];
-                    x[c] = acc * dg[c];
-                }
-#pragma unroll
-                for (int c = 0; c < kNB; ++c)
-                    if (c < kb) rp[c] = x[c];
-            }
-        }
-        grid.sync();
-        // Phase C: trailing tiles (ti, tj), tj <= ti, relative to block k+1.
-        // CTA 0 updates only tile 0, the next diagonal block, and factors it
-        // (look-ahead); the other CTAs share the remaining tiles.
-        const int tn = nblk - k - 1;
-        const int ntiles = tn * (tn + 1) / 2;
-        const int first = (G == 1) ? 0 : (blockIdx.x == 0 ? 0 : blockIdx.x);
-        const int stride = (G == 1) ? 1 : (blockIdx.x == 0 ? ntiles : G - 1);
-        for (int t = first; t < ntiles; t += stride) {
-            int ti = 0;
-            while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-            const int tj = t - ti * (ti + 1) / 2;
-            const int i0 = r0 + ti * kNB, j0 = r0 + tj * kNB;
-            const int r = threadIdx.x / 8, c4 = (threadIdx.x % 8) * 4;
-            T va[4], vb[4], vf[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = threadIdx.x + q * kThreads;
-                const int rr = e >> 5, m = e & 31;
-                va[q] = (i0 + rr < n && m < kb) ? ldg2(F + (int64_t)(i0 + rr) * n + k0 + m) : T(0);
-                vb[q] = (j0 + rr < n && m < kb) ? ldg2(F + (int64_t)(j0 + rr) * n + k0 + m) : T(0);
-            }
-            const int row = i0 + r;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int col = j0 + c4 + q;
-                vf[q] = (row < n && col < n) ? ldg2(F + (int64_t)row * n + col) : T(0);
-            }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = threadIdx.x + q * kThreads;
-                sa[e >> 5][e & 31] = va[q];
-                sb[e >> 5][e & 31] = vb[q];
-            }
-            __syncthreads();
-            T acc0 = T(0), acc1 = T(0), acc2 = T(0), acc3 = T(0);
-#pragma unroll 8
-            for (int m = 0; m < kNB; ++m) {
-                const T av = sa[r][m];
-                acc0 += av * sb[c4][m];
-                acc1 += av * sb[c4 + 1][m];
-                acc2 += av * sb[c4 + 2][m];
-                acc3 += av * sb[c4 + 3][m];
-            }
-            const T accs[4] = {acc0, acc1, acc2, acc3};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int col = j0 + c4 + q;
-                if (row < n && col < n && (ti != tj || col <= row)) F[(int64_t)row * n + col] = vf[q] - accs[q];
-            }
-            __syncthreads();
-            if (t == 0) {
-                if (!factor_diag<T>(n, F, r0, eps, sa, dg) && threadIdx.x == 0) st->solve_ok = 0;
-            }
-        }
-        grid.sync();
-    }
-}
-
-// D_k = L_kk^-1 for every 32 x 32 diagonal block, a CTA per block:
-// X = I, then per column k  X[k,:] /= L_kk and X[i,:] -= L_ik X[k,:] (i > k).
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_diag_inverses(int n, const T* __restrict__ F, T* D,
-                                                            const LmState* st) {
-    __shared__ T l[kNB][kNB + 1];
-    __shared__ T x[kNB][kNB + 1];
-    if (!st->solve_ok || st->skip_factor) return;
-    const int k0 = blockIdx.x * kNB, b = min(kNB, n - k0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        const int i = e >> 5, m = e & 31;
-        l[i][m] = (i < b && m < b) ? F[(int64_t)(k0 + i) * n + k0 + m] : (i == m ? T(1) : T(0));
-        x[i][m] = (i == m) ? T(1) : T(0);
-    }
-    __syncthreads();
-    for (int k = 0; k < kNB; ++k) {
-        const T inv = T(1) / l[k][k];
-        if (threadIdx.x < kNB) x[k][threadIdx.x] *= inv;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = threadIdx.x + q * kThreads;
-            const int i = e >> 5, c = e & 31;
-            if (i > k) x[i][c] -= l[i][k] * x[k][c];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        const int i = e >> 5, c = e & 31;
-        D[(int64_t)blockIdx.x * kNB * kNB + e] = (i < b && c < b) ? x[i][c] : T(0);
-    }
 }
 
 // Every |L_ii| must exceed 1e-7 max |L_ii|.
@@ -481,26 +269,11 @@ static int cluster_size() {
     return c;
 }
 
-template <typename TS, typename TF>
-cudaError_t launch_factor(int n, const TS* S, TF* F, TF* D, LmState* st, cudaStream_t s) {
+cudaError_t launch_factor(int n, const double* S, double* F, double* D, void* fx, LmState* st, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    const int64_t nn = (int64_t)n * n;
-    k_diag_max<TS><<<1, kThreads, 0, s>>>(n, S, st, 1e-14, 0); note_launch();
-    k_convert<TS, TF><<<grid_for(nn), kThreads, 0, s>>>(nn, S, F); note_launch();
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int nblk = (n + kNB - 1) / kNB;
-    int blocks = sms;  // one CTA per SM, all co-resident
-    if (blocks > nblk * (nblk + 1) / 2 + 1) blocks = nblk * (nblk + 1) / 2 + 1;
-    if (blocks < 1) blocks = 1;
-    int nn_i = n;
-    void* args[] = {(void*)&nn_i, (void*)&F, (void*)&st};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_chol_coop<TF>, dim3(blocks), dim3(kThreads), args, 0, s);
+    const cudaError_t e = launch_chol_fx(n, S, F, D, fx, st, s);
     if (e != cudaSuccess) return e;
-    note_launch();
-    k_check_solve_eps<TF><<<1, kThreads, 0, s>>>(n, F, st); note_launch();
-    k_diag_inverses<TF><<<nblk, kThreads, 0, s>>>(n, F, D, st); note_launch();
+    k_check_solve_eps<double><<<1, kThreads, 0, s>>>(n, F, st); note_launch();
     return cudaGetLastError();
 }
 
@@ -603,21 +376,15 @@ cudaError_t launch_solve_refine(int n, const TS* S, const TF* F, const TF* D, co
     return cudaSuccess;
 }
 
-template <typename TS, typename TF>
-cudaError_t launch_reduced_solve(int n, const TS* S, TF* F, TF* D, const double* bs, double* x, double* work,
-                                 LmState* st, int refine_iters, double tol, cudaStream_t s) {
-    cudaError_t e = launch_factor<TS, TF>(n, S, F, D, st, s);
+cudaError_t launch_reduced_solve(int n, const double* S, double* F, double* D, void* fx, const double* bs, double* x,
+                                 double* work, LmState* st, cudaStream_t s) {
+    const cudaError_t e = launch_factor(n, S, F, D, fx, st, s);
     if (e != cudaSuccess) return e;
-    return launch_solve_refine<TS, TF>(n, S, F, D, bs, x, work, st, refine_iters, tol, s);
+    return launch_solve_refine<double, double>(n, S, F, D, bs, x, work, st, 0, 0.0, s);
 }
 
-#define ZS_INST(TS, TF)                                                                                        \
-    template cudaError_t launch_factor<TS, TF>(int, const TS*, TF*, TF*, LmState*, cudaStream_t);               \
-    template cudaError_t launch_solve_refine<TS, TF>(int, const TS*, const TF*, const TF*, const double*, double*, \
-                                                     double*, LmState*, int, double, cudaStream_t);             \
-    template cudaError_t launch_reduced_solve<TS, TF>(int, const TS*, TF*, TF*, const double*, double*, double*, \
-                                                      LmState*, int, double, cudaStream_t);
-ZS_INST(double, double)
-#undef ZS_INST
+template cudaError_t launch_solve_refine<double, double>(int, const double*, const double*, const double*,
+                                                         const double*, double*, double*, LmState*, int, double,
+                                                         cudaStream_t);
 
 }  // namespace zs

@@ -23,10 +23,12 @@ namespace {
 constexpr int kMaxN = ZS_NOALLOC_MAX_N;
 constexpr size_t kBlocks = (kMaxN + 31) / 32;
 constexpr size_t kStateDoubles = (sizeof(zs::LmState) + sizeof(double) - 1) / sizeof(double);
-// A and F (n x n each), D (32 x 32 per diagonal block), b, x, the solve
-// vectors (4n + 256) and the status word, all in doubles.
+// The factor's workspace, A and F (n x n each), D (32 x 32 per diagonal
+// block), b, x, the solve vectors (4n + 256) and the status word, all in
+// doubles.
+constexpr size_t kFxDoubles = (zs::chol_fx_bytes(kMaxN) + 255) / 256 * 32;
 constexpr size_t kScratchDoubles =
-    2 * (size_t)kMaxN * kMaxN + kBlocks * 1024 + 2 * (size_t)kMaxN + (4 * (size_t)kMaxN + 256) + kStateDoubles;
+    kFxDoubles + 2 * (size_t)kMaxN * kMaxN + kBlocks * 1024 + 2 * (size_t)kMaxN + (4 * (size_t)kMaxN + 256) + kStateDoubles;
 
 __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -60,7 +62,7 @@ extern "C" int zs_dense_cholesky_solve_noalloc(const double* A, int n, const dou
     }
     double* base = g_scratch_ptr[dev];
     const size_t nn = (size_t)n * n;
-    double* dA = base;
+    double* dA = base + kFxDoubles;  // (before it: the factor's workspace)
     double* dF = dA + nn;
     double* dD = dF + nn;
     double* db = dD + 1024 * (size_t)((n + 31) / 32);
@@ -77,7 +79,7 @@ extern "C" int zs_dense_cholesky_solve_noalloc(const double* A, int n, const dou
         (e = cudaMemcpyAsync(dA, A, nn * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(db, b, n * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return fail(e);
-    if ((e = zs::launch_reduced_solve<double, double>(n, dA, dF, dD, db, dx, dwork, st, 0, 0.0, s)) != cudaSuccess)
+    if ((e = zs::launch_reduced_solve(n, dA, dF, dD, base, db, dx, dwork, st, s)) != cudaSuccess)
         return fail(e);
     zs::LmState out;
     if ((e = cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -88,5 +90,5 @@ extern "C" int zs_dense_cholesky_solve_noalloc(const double* A, int n, const dou
     if (L)
         for (int i = 0; i < n; ++i)
             for (int j = i + 1; j < n; ++j) L[(size_t)i * n + j] = 0.0;
-    return out.solve_ok ? ZS_OK : ZS_ERR_CHOLESKY;
+    return out.timeout ? ZS_ERR_TIMEOUT : (out.solve_ok ? ZS_OK : ZS_ERR_CHOLESKY);
 }
