@@ -985,7 +985,6 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
     W.bs = dalloc<double>(n, own);
     if (!batched) {
         W.F = dalloc<char>(ts * (size_t)n * n, own);
-        W.D = dalloc<char>(ts * 1024 * (size_t)((n + 31) / 32), own);
         W.work = dalloc<double>(4 * (size_t)n + 256, own);
         if (h->tsize == 4) {
             W.X = dalloc<char>(ts * (size_t)n * n, own);
@@ -1142,7 +1141,7 @@ void system_solve(zs_ba_handle* h) {
             ZS_CUDA(launch_preconditioner(P.n, W.S, (float*)W.F, (float*)W.X, (float*)W.XT, W.tc_scratch,
                                           W.tc_streams, h->st, kPreconditionerShift, W.dag_flags, &W.dag_epoch, s));
         else
-            ZS_CUDA(launch_factor(P.n, W.S, (double*)W.F, (double*)W.D, W.fx, h->st, s));
+            ZS_CUDA(launch_chol_fx(P.n, W.S, (double*)W.F, W.fx, h->st, s));
     }
     {
         PhaseScope ps(h->timer, ZS_PHASE_TRISOLVE, s);
@@ -1152,8 +1151,7 @@ void system_solve(zs_ba_handle* h) {
             // back-substitution
             ZS_CUDA(launch_pcg(P, W, h->st, std::max(0, h->opt.refine_iterations), h->opt.refine_tolerance, s));
         } else {
-            ZS_CUDA((launch_solve_refine<double, double>(P.n, W.S, (const double*)W.F, (const double*)W.D, W.bs,
-                                                         W.delta, W.work, h->st, 0, 0.0, s)));
+            ZS_CUDA(launch_trisolve(P.n, (const double*)W.F, W.bs, W.delta, W.work, h->st, s));
         }
     }
     if constexpr (sizeof(T) == 8) {
@@ -1716,7 +1714,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
         ZS_CUDA(cudaMemcpyAsync(h->st, &init, sizeof(LmState), cudaMemcpyHostToDevice, s));
         launch_invert_w<double>(P, W, h->st, s);
         launch_schur<double>(P, W, h->st, s);
-        ZS_CUDA(launch_factor(n, W.S, (double*)W.F, (double*)W.D, W.fx, h->st, s));
+        ZS_CUDA(launch_chol_fx(n, W.S, (double*)W.F, W.fx, h->st, s));
         read_state(h);
         if (!h->st_host->solve_ok) {
             status = h->st_host->timeout ? ZS_ERR_TIMEOUT : ZS_ERR_CHOLESKY;
@@ -1742,8 +1740,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 if (Xi) {
                     launch_adj_apply_inverse(n, Xi, XiT, W.bs, XiT + (size_t)n * n, W.delta, s);
                 } else {
-                    ZS_CUDA((launch_solve_refine<double, double>(n, W.S, (const double*)W.F, (const double*)W.D,
-                                                                 W.bs, W.delta, W.work, h->st, 0, 0.0, s)));
+                    ZS_CUDA(launch_trisolve(n, (const double*)W.F, W.bs, W.delta, W.work, h->st, s));
                 }
                 launch_backsub<double>(P, W, h->st, s);
                 launch_adj_copy(N, W.delta, out, s);
@@ -1867,9 +1864,8 @@ int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* Lou
         std::vector<double> Lh;
         if (precision == ZS_PRECISION_FP64) {
             double* dF = dalloc<double>(nn, owned);
-            double* dD = dalloc<double>(1024 * (size_t)((n + 31) / 32), owned);
             void* dfx = dalloc<char>(chol_fx_bytes(n), owned);
-            ZS_CUDA(launch_reduced_solve(n, dA, dF, dD, dfx, db, dx, dwork, st, s));
+            ZS_CUDA(launch_reduced_solve(n, dA, dF, dfx, db, dx, dwork, st, s));
             if (Lout) {
                 Lh.resize(nn);
                 ZS_CUDA(cudaMemcpyAsync(Lh.data(), dF, nn * sizeof(double), cudaMemcpyDeviceToHost, s));

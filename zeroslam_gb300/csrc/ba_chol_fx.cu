@@ -67,7 +67,6 @@ struct Fx {
     int n, N;
     const double* S;
     double* F;
-    double* D;    // [ceil(n / 32)][32 x 32] inverses of the diagonal blocks
     int2* Q;      // tiles (i, j), i >= j, at (i (i + 1) / 2 + j) T^2: (a0, a1) of L's entries in panels of 32
                   // columns (diagonal tiles unused)
     int2* G;      // per diagonal tile kBlocks<T> 32 x 32 blocks: scaled inverse, L (T = 64: X_11, L_21, L_11, L_22, X_22)
@@ -307,19 +306,16 @@ __device__ __noinline__ int eliminate(Smem<T>& sm, const double* C, int cl, int 
     return 1;
 }
 
-// The diagonal block's L (zeros above the diagonal) into F and its inverse
-// into D. k0: the block's first row.
+// The diagonal block's L (zeros above the diagonal) into F. k0: its first row.
 template <int T>
 __device__ void store_block(const Fx& d, const Smem<T>& sm, int k0) {
     const int kb = min(kE, d.n - k0);
 #pragma unroll
     for (int m = 0; m < kE * kE / kFxThreads; ++m) {
         const int el = threadIdx.x + m * kFxThreads, r = el >> 5, c = el & 31;
-        const bool in = r < kb && c < kb;
-        if (in)
+        if (r < kb && c < kb)
             d.F[(int64_t)(k0 + r) * d.n + k0 + c] =
                 c < r ? sm.lraw[r * kEL + c] * sm.rs[c] : (c == r ? sm.piv[r] * sm.rs[r] : 0.0);
-        d.D[(int64_t)(k0 / kE) * kE * kE + el] = in ? sm.x[r * kEL + c] : 0.0;
     }
 }
 
@@ -518,7 +514,7 @@ __device__ bool accumulate(const Fx& d, int i, int j, Smem<T>& sm, Acc<T / 16, T
 }
 
 // The diagonal tile jb from its FP64 lower triangle in sm.c(): factor, scaled
-// blocks, L and D.
+// blocks and L.
 template <int T>
 __device__ bool finish_diag(const Fx& d, int jb, int task, Smem<T>& sm, int bad) {
     constexpr int CL = T + 1;
@@ -838,7 +834,7 @@ cudaError_t launch_fx(Fx& d, int tasks, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t launch_chol_fx(int n, const double* S, double* F, double* D, void* work, LmState* st, cudaStream_t s) {
+cudaError_t launch_chol_fx(int n, const double* S, double* F, void* work, LmState* st, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     static const int stall = stall_task_from_env();
     const FxLayout l = fx_layout(n);
@@ -848,7 +844,6 @@ cudaError_t launch_chol_fx(int n, const double* S, double* F, double* D, void* w
     d.N = l.N;
     d.S = S;
     d.F = F;
-    d.D = D;
     d.Q = reinterpret_cast<int2*>(w);
     d.G = reinterpret_cast<int2*>(w + l.g);
     int* e = reinterpret_cast<int*>(w + l.e);

@@ -138,10 +138,9 @@ struct DevWork {
     double* b = nullptr;       // [n + 3L] gradient vector (poses then landmarks)
     double* S = nullptr;       // [n*n] reduced camera matrix, FP64 in both forms
     void* F = nullptr;         // [n*n] Cholesky factor (lower): double (plain form) or float (mixed)
-    void* D = nullptr;         // [ceil(n/32)*1024] T, inverses of F's diagonal blocks
     void* fx = nullptr;        // plain form: workspace of the factor, chol_fx_bytes(n)
     double* bs = nullptr;      // [n]
-    double* work = nullptr;    // [4n + 256] triangular-solve and refinement vectors
+    double* work = nullptr;    // [4n + 256] triangular-solve vectors
     void* X = nullptr;         // mixed form: [n*n] L^-1 (lower)
     void* XT = nullptr;        // mixed form: [n*n] (L^-1)^T (upper)
     int* dag_flags = nullptr;  // mixed form: [dag_flag_ints(n)] tile flags of the preconditioner's launch
@@ -368,20 +367,14 @@ void launch_match(const uint8_t* lhs, int n_lhs, const uint8_t* rhs, int n_rhs, 
                   unsigned long long* part, unsigned long long* out, cudaStream_t s);
 
 // ---- dense reduced system (ba_cholesky.cu) ----
-// launch_factor: S (n x n row-major, its lower triangle read) -> F = L (lower
-// triangle written) and D = the inverses of L's 32 x 32 diagonal blocks
-// ([ceil(n/32) * 1024]); fx: chol_fx_bytes(n), 16-byte aligned; sets
-// st->solve_ok = 0 on a failed pivot or solve test (and st->timeout when a
-// bounded wait ran out).
-// launch_solve_refine: x = (L L^T)^-1 bs, then up to refine_iters FP64
-// refinement sweeps against S until ||bs - S x|| <= tol ||bs||. work needs
-// 4n + 16 doubles. Both return the launch error, if any.
-cudaError_t launch_factor(int n, const double* S, double* F, double* D, void* fx, LmState* st, cudaStream_t s);
-template <typename TS, typename TF>
-cudaError_t launch_solve_refine(int n, const TS* S, const TF* F, const TF* D, const double* bs, double* x,
-                                double* work, LmState* st, int refine_iters, double tol, cudaStream_t s);
-cudaError_t launch_reduced_solve(int n, const double* S, double* F, double* D, void* fx, const double* bs, double* x,
-                                 double* work, LmState* st, cudaStream_t s);
+// x = (L L^T)^-1 bs with L L^T = S: launch_chol_fx, then launch_trisolve. fx:
+// chol_fx_bytes(n), 16-byte aligned; work: 2n + 2 doubles.
+cudaError_t launch_reduced_solve(int n, const double* S, double* F, void* fx, const double* bs, double* x, double* work,
+                                 LmState* st, cudaStream_t s);
+// x = (L L^T)^-1 b (ba_trisolve.cu); st->solve_ok = 0 where L fails the
+// reference's solve test. Returns at once when st->solve_ok is clear.
+cudaError_t launch_trisolve(int n, const double* F, const double* b, double* x, double* work, LmState* st,
+                            cudaStream_t s);
 
 // ---- FP64 factor (ba_chol_fx.cu) ----
 // The tile edge: up to kFxSmallN the chain of diagonal tiles bounds the launch
@@ -405,7 +398,9 @@ constexpr FxLayout fx_layout(int n) {
     return l;
 }
 constexpr size_t chol_fx_bytes(int n) { return fx_layout(n > 0 ? n : 1).bytes; }
-cudaError_t launch_chol_fx(int n, const double* S, double* F, double* D, void* work, LmState* st, cudaStream_t s);
+// S (n x n row-major, its lower triangle read) -> F = L (lower triangle
+// written); st->solve_ok = 0 on a failed pivot.
+cudaError_t launch_chol_fx(int n, const double* S, double* F, void* work, LmState* st, cudaStream_t s);
 
 // ---- mixed form: the preconditioner (ba_chol_dag.cu) ----
 // F (n x n FP32, the matrix) -> L in F's lower triangle (zeros above the

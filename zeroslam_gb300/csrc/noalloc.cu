@@ -8,7 +8,7 @@
 // framework's memory pool) so that a private cudaMalloc is not allowed.
 //
 // How: every device buffer the solve needs (device copies of A and b, the
-// factor, the diagonal-block inverses, the solve vectors and the status
+// factor and its workspace, the solve vectors and the status
 // word) is carved out of one file-scope __device__ array of fixed size,
 // sized for n <= ZS_NOALLOC_MAX_N. The array exists once per device that
 // loads this library and stays allocated until the process exits.
@@ -21,14 +21,12 @@
 namespace {
 
 constexpr int kMaxN = ZS_NOALLOC_MAX_N;
-constexpr size_t kBlocks = (kMaxN + 31) / 32;
 constexpr size_t kStateDoubles = (sizeof(zs::LmState) + sizeof(double) - 1) / sizeof(double);
-// The factor's workspace, A and F (n x n each), D (32 x 32 per diagonal
-// block), b, x, the solve vectors (4n + 256) and the status word, all in
-// doubles.
+// The factor's workspace, A and F (n x n each), b, x, the solve vectors and
+// the status word, all in doubles.
 constexpr size_t kFxDoubles = (zs::chol_fx_bytes(kMaxN) + 255) / 256 * 32;
 constexpr size_t kScratchDoubles =
-    kFxDoubles + 2 * (size_t)kMaxN * kMaxN + kBlocks * 1024 + 2 * (size_t)kMaxN + (4 * (size_t)kMaxN + 256) + kStateDoubles;
+    kFxDoubles + 2 * (size_t)kMaxN * kMaxN + 2 * (size_t)kMaxN + (4 * (size_t)kMaxN + 256) + kStateDoubles;
 
 __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -64,8 +62,7 @@ extern "C" int zs_dense_cholesky_solve_noalloc(const double* A, int n, const dou
     const size_t nn = (size_t)n * n;
     double* dA = base + kFxDoubles;  // (before it: the factor's workspace)
     double* dF = dA + nn;
-    double* dD = dF + nn;
-    double* db = dD + 1024 * (size_t)((n + 31) / 32);
+    double* db = dF + nn;
     double* dx = db + n;
     double* dwork = dx + n;
     zs::LmState* st = reinterpret_cast<zs::LmState*>(base + (kScratchDoubles - kStateDoubles));
@@ -79,7 +76,7 @@ extern "C" int zs_dense_cholesky_solve_noalloc(const double* A, int n, const dou
         (e = cudaMemcpyAsync(dA, A, nn * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(db, b, n * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return fail(e);
-    if ((e = zs::launch_reduced_solve(n, dA, dF, dD, base, db, dx, dwork, st, s)) != cudaSuccess)
+    if ((e = zs::launch_reduced_solve(n, dA, dF, base, db, dx, dwork, st, s)) != cudaSuccess)
         return fail(e);
     zs::LmState out;
     if ((e = cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
