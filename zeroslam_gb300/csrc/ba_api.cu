@@ -975,7 +975,13 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
         W.jp_pm = dalloc<float4>(3 * (size_t)M, own);
         W.hll_inv_f = dalloc<float>(12 * (size_t)std::max(L, 1), own);
     }
-    else W.lm_part = dalloc<char>(ts * 12 * M, own);  // record-major, 9 values padded to 12
+    else {
+        W.lm_part = dalloc<char>(ts * 12 * M, own);  // record-major, 9 values padded to 12
+        W.fxw = dalloc<int4>(10 * (size_t)M, own);
+        W.fxh = dalloc<int4>(10 * (size_t)M, own);
+        W.row_exp = dalloc<int>(12 * (size_t)K, own);
+        W.lm_exp = dalloc<int>((size_t)std::max(L, 1), own);
+    }
     W.pose_part = dalloc<char>(ts * 28 * M, own);  // record-major, 27 values padded to 28
     W.hpp = dalloc<double>((size_t)K * 36, own);
     W.hll = dalloc<double>((size_t)L * 9, own);
@@ -1010,6 +1016,7 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
     W.red = dalloc<double>(std::max<size_t>(kReduceBlocks * 4 + 16, (size_t)P.nochunks), own);
     W.ired = dalloc<int32_t>(kReduceBlocks, own);
     ZS_CUDA(cudaMemsetAsync(W.hll_inv, 0, sizeof(double) * 9 * (size_t)std::max(L, 1), s));
+    if (W.lm_exp) ZS_CUDA(cudaMemsetAsync(W.lm_exp, 0, sizeof(int) * (size_t)std::max(L, 1), s));
     ZS_CUDA(cudaMemsetAsync(W.delta, 0, sizeof(double) * std::max<size_t>(1, (size_t)n + 3 * (size_t)L), s));
     ZS_CUDA(cudaStreamSynchronize(s));
     ZS_CUDA(cudaGetLastError());

@@ -69,14 +69,15 @@ __device__ inline double cta_max(double v, double* sh) {
 
 // matrix::invert<3> on H_ll + lambda_w I, as k_invert (source/matrix.hpp:749-774).
 __global__ void __launch_bounds__(kThreads) k_binvert(DevProblem P, const double* __restrict__ hll, double* hinv,
-                                                      float* hinv_f, const LmState* __restrict__ st,
-                                                      const WinCtl* __restrict__ ctl) {
+                                                      float* hinv_f, int* lm_exp, int* row_exp,
+                                                      const LmState* __restrict__ st, const WinCtl* __restrict__ ctl) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row_exp && l < 12 * P.K) row_exp[l] = kRowExpEmpty;
     if (l >= P.L) return;
     const int w = P.lm_win[l];
     if (!ctl[w].active) return;
     landmark_inverse(hll + (int64_t)l * 9, st[w].lambda, P.lm_fixed[l] != 0, hinv + (int64_t)l * 9,
-                     hinv_f ? hinv_f + (int64_t)l * 12 : nullptr);
+                     hinv_f ? hinv_f + (int64_t)l * 12 : nullptr, lm_exp ? lm_exp + l : nullptr);
 }
 
 // S_w = blockdiag(H_pp) + lambda_w I; blockIdx.y = window.
@@ -647,8 +648,9 @@ cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, con
                                cudaStream_t s) {
     launch_linearize<T>(P, W, s);
     if (P.L > 0) {
-        k_binvert<<<grid_for(P.L), kThreads, 0, s>>>(P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr,
-                                                     B.st, B.ctl);
+        k_binvert<<<grid_for(std::max(P.L, W.row_exp ? 12 * P.K : 0)), kThreads, 0, s>>>(
+            P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, W.lm_exp, W.row_exp,
+            B.st, B.ctl);
         note_launch();
     }
     launch_w<T>(P, W, s);

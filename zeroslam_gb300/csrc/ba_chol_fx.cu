@@ -46,16 +46,16 @@
 
 #include <cstdlib>
 
+#include "ba_fixed.cuh"
 #include "ba_internal.h"
 
 namespace zs {
 
 namespace {
 
-using ll = long long;
+using namespace fixed;
 
 constexpr int kFxThreads = 256;
-constexpr int kLow = 30;                        // bits of a0
 constexpr int kFrac = 60;                       // q = scaled value x 2^kFrac
 constexpr int kAccFrac = 2 * (kFrac - kLow);    // the sum of a1 b1 is in units of 2^-kAccFrac
 constexpr ll kMaxQ = 3ll << (kFrac - 1);        // 1.5
@@ -98,35 +98,8 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// 2^p as a double, p in [-1022, 1023].
-__device__ __forceinline__ double pow2(int p) { return __longlong_as_double((ll)(p + 1023) << 52); }
-
-// round(v 2^sh) to nearest; bad is set where that is above kMaxQ or not finite.
-__device__ __forceinline__ ll quantize(double v, int sh, int& bad) {
-    const ll bits = __double_as_longlong(v);
-    const int ex = (int)((bits >> 52) & 0x7ff);
-    const ll m = (bits & ((1ll << 52) - 1)) | (ex ? 1ll << 52 : 0);
-    const int s = (ex ? ex : 1) - 1075 + sh;  // v 2^sh = m 2^s
-    ll q;
-    if (s >= 0) {
-        q = m << min(s, 10);
-    } else {
-        q = s > -55 ? (m + (1ll << (-s - 1))) >> -s : 0;
-    }
-    if (ex == 0x7ff || q > kMaxQ) bad = 1;
-    return bits < 0 ? -q : q;
-}
-
-__device__ __forceinline__ int2 split(ll q) {
-    const ll a1 = (q + (1ll << (kLow - 1))) >> kLow;
-    return make_int2((int)(q - (a1 << kLow)), (int)a1);
-}
-
-// x 2^s, s of either sign (to nearest below zero).
-__device__ __forceinline__ ll shift(ll x, int s) {
-    if (s >= 0) return x << min(s, 63);
-    return s > -63 ? (x + (1ll << (-s - 1))) >> -s : 0;
-}
+// As fixed::quantize, at most kMaxQ.
+__device__ __forceinline__ ll quantize(double v, int sh, int& bad) { return fixed::quantize(v, sh, kMaxQ, bad); }
 
 template <int RA, int RB>
 struct Acc {
@@ -328,13 +301,13 @@ __device__ void scale_blocks(const Fx& d, Smem<T>& sm, int k0, int2* X, int2* Lb
     const int t = threadIdx.x, r = t >> 3, q = t & 7;
     const int er = d.e[k0 + r];
     double v[4];
-    int em[4], top = -4000;
+    int em[4], top = -8192;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         const int j = 8 * m + q;
         v[m] = sm.x[r * kEL + j];
         em[m] = d.e[k0 + j];
-        if (v[m] != 0.0) top = max(top, (int)((__double_as_longlong(v[m]) >> 52) & 0x7ff) - 1022 + em[m]);
+        top = max(top, exponent(v[m]) + em[m]);
     }
 #pragma unroll
     for (int off = 1; off < 8; off <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, off));

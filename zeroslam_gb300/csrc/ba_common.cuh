@@ -229,9 +229,11 @@ __device__ inline double cost_fast(const double* __restrict__ a, const double* _
 // (source/matrix.hpp:749-774): fixed landmarks and singular blocks
 // (|det| <= 1e-12 max|a|^3) get a zero inverse, as solve_linear_system
 // ignores the failed inversion (source/factor_graph.hpp:763). of (optional,
-// mixed form) also receives the inverse in FP32, padded to 12 floats.
+// mixed form) also receives the inverse in FP32, padded to 12 floats; oe
+// (optional, plain form) s, about half the exponent of the inverse's largest
+// entry: H_pl 2^s and H_pl H_ll^-1 2^-s are then of like size.
 __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double lam, bool fixed, double* o,
-                                        float* of) {
+                                        float* of, int* oe) {
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (!fixed) {
         double a[9];
@@ -258,6 +260,11 @@ __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) o[i] = v[i];
+    if (oe) {
+        const double m = fmax(fabs(v[0]), fmax(fabs(v[4]), fabs(v[8])));
+        const int e = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
+        *oe = e == 0 || e == 0x7ff ? 0 : (e - 1022) >> 1;
+    }
     if (of) {
         float4* f = reinterpret_cast<float4*>(of);
         f[0] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);

@@ -99,6 +99,9 @@ struct DevProblem {
     int32_t* lmch_l = nullptr;     // [nlmch+1]
 };
 
+// DevWork::row_exp of a row without entries.
+constexpr int kRowExpEmpty = -4096;
+
 // At most this many observations per operator chunk (a warp's share).
 constexpr int kOpChunk = 64;
 
@@ -126,6 +129,10 @@ struct DevWork {
     void* W = nullptr;         // [M*RS] T, pose-major positions
     double* pose_aux = nullptr; // [K*24] mixed form: per-pose sandwich matrix, translation, rotation
     double* partial = nullptr; // [nsegs*36] Schur segment sums (FP64)
+    int4* fxw = nullptr;       // plain form: [M*10] W in fixed point, pose-major positions
+    int4* fxh = nullptr;       // plain form: [M*10] H_pl in fixed point
+    int* row_exp = nullptr;    // plain form: [12K] exponents of the scales of each pose's rows: H_pl (6K), W (6K)
+    int* lm_exp = nullptr;     // plain form: [L] exponents of the landmarks' balance
     void* lm_part = nullptr;   // plain form: [M*12] per-observation landmark records (9 used)
     ObsJac* jac = nullptr;     // mixed form: [M] per-observation Jacobian records
     float4* jp_pm = nullptr;   // mixed form: [3M] J_p of each record again, pose-major positions, three planes

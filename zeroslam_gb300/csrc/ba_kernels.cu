@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "ba_df.cuh"
+#include "ba_fixed.cuh"
 #include "ba_internal.h"
 
 namespace zs {
@@ -609,22 +610,88 @@ __global__ void __launch_bounds__(kThreads) k_reduce_pose_runs(DevProblem P, con
     }
 }
 
-// Damped 3x3 landmark inverses (landmark_inverse).
+// Damped 3x3 landmark inverses (landmark_inverse); the plain form's row_exp is
+// cleared for k_w on the way.
 __global__ void __launch_bounds__(kThreads) k_invert(DevProblem P, const double* __restrict__ hll, double* hinv,
-                                                     float* hinv_f, const LmState* st) {
+                                                     float* hinv_f, int* lm_exp, int* row_exp, const LmState* st) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row_exp && l < 12 * P.K) row_exp[l] = kRowExpEmpty;
     if (l >= P.L) return;
     landmark_inverse(hll + (int64_t)l * 9, st->lambda, P.lm_fixed[l] != 0, hinv + (int64_t)l * 9,
-                     hinv_f ? hinv_f + (int64_t)l * 12 : nullptr);
+                     hinv_f ? hinv_f + (int64_t)l * 12 : nullptr, lm_exp ? lm_exp + l : nullptr);
 }
 
 // W = H_pl H_ll^-1 per block. Mixed form: the FP32 inverses (hinv_f, 12
-// floats per landmark) and 16-byte record loads and stores.
+// floats per landmark) and 16-byte record loads and stores. Plain form: also
+// the exponents of each pose row's largest entries (row_exp, cleared before),
+// of H_pl 2^s and of W 2^-s, s = lm_exp of the landmark: the scales of the
+// fixed-point records.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_w(DevProblem P, const T* __restrict__ hpl, const double* __restrict__ hinv,
-                                                const float* __restrict__ hinv_f, T* __restrict__ W) {
+                                                const float* __restrict__ hinv_f, T* __restrict__ W,
+                                                const int* __restrict__ lm_exp, int* row_exp) {
     constexpr int RS = RecStride<T>::value;
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // pose-major position
+    if constexpr (sizeof(T) == 8) {
+        // (every lane stays for the warp's maxima)
+        const bool in = q < P.M;
+        const int64_t o = P.pose_obs[in ? q : P.M - 1];
+        const bool valid = in && P.blk_valid[o];
+        const int pose = P.obs_pose[o];
+        int eh[6], ew[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) eh[a] = ew[a] = kRowExpEmpty;
+        if (valid) {
+            const int l = P.obs_lm[o];
+            const double* I = hinv + (int64_t)l * 9;
+            const int s = lm_exp[l];
+            double iv[9];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) iv[i] = I[i];
+            const double2* h2 = reinterpret_cast<const double2*>(hpl + q * RS);
+            double2* w2 = reinterpret_cast<double2*>(W + q * RS);
+            double h[18], w[18];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                const double2 t = __ldg(h2 + i);
+                h[2 * i] = t.x;
+                h[2 * i + 1] = t.y;
+            }
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                int mh = -4096, mw = -4096;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    w[a * 3 + c] = h[a * 3] * iv[c] + h[a * 3 + 1] * iv[3 + c] + h[a * 3 + 2] * iv[6 + c];
+                    mh = max(mh, fixed::exponent(h[a * 3 + c]));
+                    mw = max(mw, fixed::exponent(w[a * 3 + c]));
+                }
+                // (values that are not finite stay recognisable)
+                eh[a] = mh > 1024 ? 8192 : mh + s;
+                ew[a] = mw > 1024 ? 8192 : mw - s;
+            }
+#pragma unroll
+            for (int i = 0; i < 9; ++i) w2[i] = make_double2(w[2 * i], w[2 * i + 1]);
+        }
+        const int first = __shfl_sync(0xffffffffu, pose, 0);
+        if (__all_sync(0xffffffffu, pose == first)) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                const int mh = __reduce_max_sync(0xffffffffu, eh[a]), mw = __reduce_max_sync(0xffffffffu, ew[a]);
+                if ((threadIdx.x & 31) == a) {
+                    atomicMax(row_exp + 6 * first + a, mh);
+                    atomicMax(row_exp + 6 * (P.K + first) + a, mw);
+                }
+            }
+        } else if (valid) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                atomicMax(row_exp + 6 * pose + a, eh[a]);
+                atomicMax(row_exp + 6 * (P.K + pose) + a, ew[a]);
+            }
+        }
+        return;
+    }
     if (q >= P.M) return;
     const int64_t o = P.pose_obs[q];
     if (!P.blk_valid[o]) return;
@@ -649,19 +716,6 @@ __global__ void __launch_bounds__(kThreads) k_w(DevProblem P, const T* __restric
         float4* w4 = reinterpret_cast<float4*>(W + q * RS);
 #pragma unroll
         for (int i = 0; i < 5; ++i) w4[i] = make_float4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-    } else {
-        const double* I = hinv + (int64_t)P.obs_lm[o] * 9;
-        T iv[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) iv[i] = (T)I[i];
-        const T* h = hpl + q * RS;
-        T* w = W + q * RS;
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-            const T h0 = h[a * 3], h1 = h[a * 3 + 1], h2 = h[a * 3 + 2];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) w[a * 3 + c] = h0 * iv[c] + h1 * iv[3 + c] + h2 * iv[6 + c];
-        }
     }
 }
 
@@ -722,57 +776,151 @@ __global__ void __launch_bounds__(kSchurThreadsF32) k_schur_segments(DevProblem 
     }
 }
 
-// The same sums in FP64. The FP64 pipe bounds them (one lane's multiply-add
-// per two cycles and SM quarter: a warp's instruction holds it for 64
-// cycles, whether its lanes are in use or not), so lanes must not idle: four
-// lanes share a triple, each the 3 x 3 quarter of its 6 x 6 product, and the
-// warp takes eight triples at a time. A segment of m triples then costs
-// 27 ceil(m / 8) multiply-adds per warp and 27 for the butterfly over the
-// eight groups; with a lane per triple it was 108 ceil(m / 32) and 64.
-__global__ void __launch_bounds__(kSchurThreadsF64) k_schur_segments_f64(DevProblem P, const double* __restrict__ W,
-                                                                         const double* __restrict__ hpl,
-                                                                         double* __restrict__ part,
-                                                                         const WinCtl* __restrict__ ctl) {
+// The plain form's sums, in fixed point on the integer pipe. An FP64
+// multiply-add holds an SM quarter's FP64 pipe for 64 cycles a warp (whether
+// its lanes are in use or not), an integer one (32 x 32 + 64 bits) takes
+// about three. So the records are held as integers (k_schur_fix): row a of
+// H_pl of pose j times 2^s and of W of pose i times 2^-s, s balancing the
+// landmark's two, over the largest entry of that row of that pose, 2^58 steps
+// each. Products and sums are exact but for the lowest half of a product; an
+// entry is rounded at 2^-59 of its row's largest. FP64 rounds each sum at
+// 2^-53 of itself; over a pair's products, of mean size 1/20 or so of the
+// largest, that is more, or as much where a pair shares only a few.
+constexpr int kSchurFrac = 58;
+constexpr int kSchurMinExp = -990;  // rows below 2^-990 (or all zero) are scaled by that: the scales stay normal
+
+// H_pl 2^s and W 2^-s of one observation in fixed point, 10 x 16 bytes each:
+// rows 0-2 and rows 3-5 of the 6 x 3 block, 9 pairs and a pad.
+__global__ void __launch_bounds__(kThreads) k_schur_fix(DevProblem P, const double* __restrict__ W,
+                                                        const double* __restrict__ hpl, const int* __restrict__ lm_exp,
+                                                        const int* __restrict__ row_exp, int4* __restrict__ fxw,
+                                                        int4* __restrict__ fxh) {
     constexpr int RS = RecStride<double>::value;
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= P.M) return;
+    const int64_t o = P.pose_obs[q];
+    if (!P.blk_valid[o]) return;
+    const int s = lm_exp[P.obs_lm[o]];
+    int bad = 0;
+    auto convert = [&](const double* src, const int* e, int sign, int4* dst) {
+        const double2* v2 = reinterpret_cast<const double2*>(src);
+        double v[18];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            const double2 t = __ldg(v2 + i);
+            v[2 * i] = t.x;
+            v[2 * i + 1] = t.y;
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            int2 p[10];
+#pragma unroll
+            for (int i = 0; i < 9; ++i)
+                p[i] = fixed::split(fixed::quantize(v[9 * half + i], kSchurFrac - max(e[3 * half + i / 3], kSchurMinExp) + sign * s,
+                                                    1ll << kSchurFrac, bad));
+            p[9] = make_int2(0, 0);
+#pragma unroll
+            for (int i = 0; i < 5; ++i) dst[5 * half + i] = make_int4(p[2 * i].x, p[2 * i].y, p[2 * i + 1].x, p[2 * i + 1].y);
+        }
+    };
+    const int pose = P.obs_pose[o];
+    convert(hpl + q * RS, row_exp + 6 * pose, 1, fxh + q * 10);
+    convert(W + q * RS, row_exp + 6 * (P.K + pose), -1, fxw + q * 10);
+}
+
+// Four lanes share a triple, each the 3 x 3 quarter of its 6 x 6 product; the
+// warp takes eight triples at a time. Sums of a lane over 8 triples (24
+// products) stay below 2^63: a1 b1 at most 2^56, a1 b0 2^57, a0 b0 >> 32 2^26;
+// the carries after them keep the total in top (units 2^8 of hi). The eight
+// groups' integers meet in a butterfly and each group converts an output or
+// two to FP64.
+__global__ void __launch_bounds__(kSchurThreadsF64) k_schur_segments_fx(DevProblem P, const int4* __restrict__ fxw,
+                                                                        const int4* __restrict__ fxh,
+                                                                        const int* __restrict__ row_exp,
+                                                                        double* __restrict__ part,
+                                                                        const WinCtl* __restrict__ ctl) {
+    using fixed::ll;
+    constexpr int kLow = fixed::kLow;
     const int lane = threadIdx.x & 31;
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (g >= P.nsegs || !schur_segment_active(P, g, ctl)) return;
-    const int r3 = 3 * ((lane >> 1) & 1), c3 = 3 * (lane & 1);  // the quarter's first row and column
-    double acc[3][3];
+    const int rh = (lane >> 1) & 1, ch = lane & 1;  // the quarter's rows and columns: the first or last three
+    ll top[9], hi[9], mid[9];
+    int lo[9];
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) acc[a][d] = 0.0;
+    for (int i = 0; i < 9; ++i) {
+        top[i] = hi[i] = mid[i] = 0;
+        lo[i] = 0;
+    }
     const int64_t t1 = P.seg_ptr[g + 1];
     int64_t t = P.seg_ptr[g] + (lane >> 2);
     int2 tr = t < t1 ? P.triples[t] : make_int2(0, 0);
-    while (t < t1) {
-        const double* wp = W + (int64_t)tr.x * RS + 3 * r3;
-        const double* hp = hpl + (int64_t)tr.y * RS + 3 * c3;
-        t += 8;
-        if (t < t1) tr = P.triples[t];
-        double w[9], h[9];
+    while (__any_sync(0xffffffffu, t < t1)) {
+#pragma unroll 1
+        for (int k = 0; k < 8 && t < t1; ++k) {
+            const int4* wp = fxw + (int64_t)tr.x * 10 + 5 * rh;
+            const int4* hp = fxh + (int64_t)tr.y * 10 + 5 * ch;
+            t += 8;
+            if (t < t1) tr = P.triples[t];
+            int2 w[10], h[10];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            w[i] = __ldg(wp + i);
-            h[i] = __ldg(hp + i);
+            for (int i = 0; i < 5; ++i) {
+                const int4 a = __ldg(wp + i), b = __ldg(hp + i);
+                w[2 * i] = make_int2(a.x, a.y);
+                w[2 * i + 1] = make_int2(a.z, a.w);
+                h[2 * i] = make_int2(b.x, b.y);
+                h[2 * i + 1] = make_int2(b.z, b.w);
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const int2 x = w[3 * a + c], y = h[3 * d + c];
+                        hi[3 * a + d] += (ll)x.y * y.y;
+                        mid[3 * a + d] += (ll)x.y * y.x;
+                        mid[3 * a + d] += (ll)x.x * y.y;
+                        lo[3 * a + d] += __mulhi(x.x, y.x);
+                    }
         }
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                acc[a][d] = fma(w[3 * a], h[3 * d], fma(w[3 * a + 1], h[3 * d + 1], fma(w[3 * a + 2], h[3 * d + 2], acc[a][d])));
+        for (int i = 0; i < 9; ++i) {
+            mid[i] += (ll)lo[i] << (32 - kLow);
+            lo[i] = 0;
+            hi[i] += mid[i] >> kLow;
+            mid[i] &= (1ll << kLow) - 1;
+            top[i] += hi[i] >> 8;
+            hi[i] &= 255;
+        }
+        __syncwarp();
     }
+    // the groups' totals: top, and hi 2^30 + mid below 2^38 each
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        ll r = (hi[i] << kLow) | mid[i];
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            top[i] += __shfl_xor_sync(0xffffffffu, top[i], off);
+            r += __shfl_xor_sync(0xffffffffu, r, off);
+        }
+        mid[i] = r;
+    }
+    const int p = P.seg_pair[g], grp = lane >> 2;
+    const int* ew = row_exp + 6 * (P.K + P.pair_i[p]) + 3 * rh;
+    const int* eh = row_exp + 6 * P.pair_j[p] + 3 * ch;
     double* out = part + g * 36;
-    __syncwarp();
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            double v = acc[a][d];
-#pragma unroll
-            for (int off = 4; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (lane < 4) out[(r3 + a) * 6 + c3 + d] = v;
+    for (int i = 0; i < 9; ++i)
+        if (grp == (i & 7)) {
+            // units of the total: 2^-(2 x 58 - 60) for hi, 2^8 of it for top, 2^-30 for r; the scales in two steps, so
+            // that neither leaves the range of a double
+            const int e1 = ew[i / 3], e2 = eh[i % 3];
+            const double v = fma((double)top[i], 256.0, (double)mid[i] * fixed::pow2(-kLow));
+            const bool ok = e1 <= 1024 && e2 <= 1024;
+            const double s1 = ok ? fixed::pow2(max(e1, kSchurMinExp) - (kSchurFrac - kLow)) : __longlong_as_double(0x7ff8000000000000ll);
+            const double s2 = ok ? fixed::pow2(max(e2, kSchurMinExp) - (kSchurFrac - kLow)) : 0.0;
+            out[(3 * rh + i / 3) * 6 + 3 * ch + i % 3] = v * s1 * s2;
         }
 }
 
@@ -1135,23 +1283,33 @@ void launch_linearize(const DevProblem& P, DevWork& W, cudaStream_t s) {
 }
 
 template <typename T>
+void launch_w(const DevProblem& P, DevWork& W, cudaStream_t s) {
+    if (P.M <= 0) return;
+    k_w<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.hll_inv_f, (T*)W.W, W.lm_exp, W.row_exp);
+    note_launch();
+    if constexpr (sizeof(T) == 8) {
+        k_schur_fix<<<grid_for(P.M), kThreads, 0, s>>>(P, (const double*)W.W, (const double*)W.hpl, W.lm_exp, W.row_exp,
+                                                       W.fxw, W.fxh);
+        note_launch();
+    }
+}
+
+template <typename T>
 void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s) {
     if (P.L > 0) {
-        k_invert<<<grid_for(P.L), kThreads, 0, s>>>(P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, st);
+        k_invert<<<grid_for(std::max(P.L, W.row_exp ? 12 * P.K : 0)), kThreads, 0, s>>>(
+            P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, W.lm_exp, W.row_exp, st);
         note_launch();
     }
-    if (P.M > 0) {
-        k_w<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.hll_inv_f, (T*)W.W);
-        note_launch();
-    }
+    launch_w<T>(P, W, s);
 }
 
 template <typename T>
 void launch_schur_pairs(const DevProblem& P, DevWork& W, const WinCtl* ctl, cudaStream_t s) {
     if (P.npairs > 0) {
         if constexpr (sizeof(T) == 8)
-            k_schur_segments_f64<<<grid_for(32 * P.nsegs, kSchurThreadsF64), kSchurThreadsF64, 0, s>>>(
-                P, (const double*)W.W, (const double*)W.hpl, W.partial, ctl);
+            k_schur_segments_fx<<<grid_for(32 * P.nsegs, kSchurThreadsF64), kSchurThreadsF64, 0, s>>>(
+                P, W.fxw, W.fxh, W.row_exp, W.partial, ctl);
         else
             k_schur_segments<<<grid_for(32 * P.nsegs, kSchurThreadsF32), kSchurThreadsF32, 0, s>>>(
                 P, (const float*)W.W, (const float*)W.hpl, W.partial, ctl);
@@ -1179,15 +1337,6 @@ void launch_bs(const DevProblem& P, DevWork& W, cudaStream_t s) {
         launch_pose_sums6(P, W.opch_sum, BsTerm<T>{(const T*)W.W, W.b}, BsOut{W.b, W.bs}, s);
     }
 }
-
-template <typename T>
-void launch_w(const DevProblem& P, DevWork& W, cudaStream_t s) {
-    if (P.M > 0) {
-        k_w<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.hll_inv_f, (T*)W.W);
-        note_launch();
-    }
-}
-
 
 template <typename T>
 void launch_backsub(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s) {
