@@ -48,9 +48,20 @@ def test_factor(zs_lib, n, kind):
     assert r <= 40 * (n + 2) * 2.0**-53 * np.linalg.norm(A, 2) * np.linalg.norm(x)
 
 
+@pytest.mark.parametrize("n", [4608, 4609, 4641, 4705])
+def test_factor_large(zs_lib, n):
+    """Either side of the change of tiles (n = 4608), and the 64-wide tiles' ragged ends."""
+    test_factor(zs_lib, n, "plain")
+
+
+@pytest.mark.parametrize("kind", ["late", "nan"])
+def test_not_positive_definite_large(zs_lib, kind):
+    test_not_positive_definite(zs_lib, kind, 4700)
+
+
 @pytest.mark.parametrize("n", [2, 40, 130, 1600])
 @pytest.mark.parametrize("kind", ["negative", "zero", "large", "correlated", "late", "nan", "inf"])
-def test_not_positive_definite(zs_lib, n, kind):
+def test_not_positive_definite(zs_lib, kind, n):
     A = _spd(n, n + 7, "scaled")
     if kind == "negative":
         A[n - 1, n - 1] *= -1
@@ -81,7 +92,7 @@ CHILD = r"""
 import numpy as np
 from zeroslam_gb300 import ba
 rng = np.random.default_rng(0)
-for n in (200, 1600):
+for n in (200, 4700):
     G = rng.normal(size=(n, n)); A = G @ G.T / n + np.eye(n); b = rng.normal(size=n)
     st = ba.dense_cholesky_status(A, b, precision=ba.FP64)
     assert st == ba.ZS_ERR_TIMEOUT, st

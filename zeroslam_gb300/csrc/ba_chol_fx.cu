@@ -4,9 +4,10 @@
 //
 // A GB300 SM quarter takes one FP64 multiply-add per two cycles, a warp's
 // instruction 64 cycles (measured, whether its lanes are in use or not), and
-// a 32 x 32 -> 64-bit integer multiply-add per 2.2. So the factor's products,
-// nearly all of its work, run in fixed point, and FP64 is kept for what is
-// sequential: the 32 x 32 diagonal blocks.
+// a 32 x 32 -> 64-bit integer multiply-add per about three. So the factor
+// runs in fixed point: its products, nearly all of its work, and the chain of
+// pivots, whose every step would otherwise wait on several FP64
+// instructions.
 //
 // Fixed point. Row r is scaled by 2^-e_r, 2^e_r >= sqrt(S_rr): for a positive
 // definite S every |L_rc| 2^-e_r <= 1, every Schur complement's entry
@@ -19,9 +20,7 @@
 // bits: unlike FP64's, the rounding of a small entry is no smaller, and over
 // the rows of a large matrix it adds up. With 2^-56 and a0 b0 dropped, the
 // step of the 6,000-row loop was 4.6 times further from 64 bits than FP64's,
-// with 2^-58 twice.)
-// The diagonal entries' differences S_rr - sum and the diagonal blocks'
-// elimination, with its pivot test, are FP64.
+// with 2^-58 twice.) A pivot is compared with 1e-14 max |S_ii| in its row's scale.
 //
 // Where a bound above does not hold, S is not positive definite and the
 // factor fails, as the pivot test of the FP64 factor would: a scaled entry
@@ -33,15 +32,14 @@
 // Tiles are T x T (32 or 64); every tile has one owner CTA that computes it
 // completely, in a fixed order, and publishes it with a flag (cleared by
 // k_fx_prepare): tile (i, j), i > j, is C_ij = S_ij - sum_{k<j} L_ik L_jk^T
-// times L_jj^-T, by products with the inverses of L_jj's 32 x 32 diagonal
-// blocks; such a product's error grows with the block's condition number, so
-// each is corrected once with its residual, L += (C - L L_kk^T) L_kk^-T. Tasks are numbered column block by column block, CTA
+// times L_jj^-T by substitution; the diagonal tile j is factored in blocks of
+// 32 columns. Tasks are numbered column block by column block, CTA
 // t mod G takes its tasks in increasing order, every dependency has a
 // smaller number and all CTAs are co-resident (cooperative launch), so the
 // lowest unfinished task can always proceed. With T = 32 the task of tile
-// (c + 1, c) also factors diagonal tile c + 1. A wait gives up after a bounded number of polls: the
-// launch is then marked aborted (every other wait returns), st->timeout set
-// and st->solve_ok cleared.
+// (c + 1, c) also factors diagonal tile c + 1. A wait gives up after a
+// bounded number of polls: the launch is then marked aborted (every other
+// wait returns), st->timeout set and st->solve_ok cleared.
 #include <cooperative_groups.h>
 
 #include <cstdlib>
@@ -57,9 +55,9 @@ using namespace fixed;
 
 constexpr int kFxThreads = 256;
 constexpr int kFrac = 60;                       // q = scaled value x 2^kFrac
-constexpr int kAccFrac = 2 * (kFrac - kLow);    // the sum of a1 b1 is in units of 2^-kAccFrac
+static_assert(2 * (kFrac - kLow) == kFrac, "sums of a1 b1 are in units of 2^-kFrac");
 constexpr ll kMaxQ = 3ll << (kFrac - 1);        // 1.5
-constexpr ll kMaxDiag = 5ll << (kAccFrac - 2);  // 1.25
+constexpr ll kMaxDiag = 5ll << (kFrac - 2);  // 1.25
 constexpr float kMaxRow = 1.25f;
 constexpr long long kSpinLimit = 1ll << 20;  // polls of one flag before a wait gives up (about a second)
 
@@ -69,9 +67,9 @@ struct Fx {
     double* F;
     int2* Q;      // tiles (i, j), i >= j, at (i (i + 1) / 2 + j) T^2: (a0, a1) of L's entries in panels of 32
                   // columns (diagonal tiles unused)
-    int2* G;      // per diagonal tile kBlocks<T> 32 x 32 blocks: scaled inverse, L (T = 64: X_11, L_21, L_11, L_22, X_22)
+    int2* G;      // per diagonal tile kBlocks<T> 32 x 32 blocks of its L (T = 64: L_11, L_21, L_22)
     const int* e; // [N T] row scales
-    int* f;       // [N T] shifts of the products with the inverses' rows
+    int4* f;      // [N T] columns' pivots: Pivot
     LmState* st;
     int* flag;    // tiles as Q: 1 once final
     int* abort;   // 1 once the launch has given up
@@ -141,10 +139,10 @@ struct Acc {
                 mid[i][j] -= c << kLow;
             }
     }
-    // the sum in units of 2^-kAccFrac, to nearest
-    __device__ __forceinline__ ll value(int i, int j) const { return hi[i][j] + ((mid[i][j] + (1ll << (kLow - 1))) >> kLow); }
-    // the same in units of 2^-kFrac
-    __device__ __forceinline__ ll value_q(int i, int j) const { return shift(value(i, j), kFrac - kAccFrac); }
+    // the sum in units of 2^-kFrac, to nearest
+    __device__ __forceinline__ ll value(int i, int j) const {
+        return hi[i][j] + ((mid[i][j] + ((ll)lo[i][j] << (32 - kLow)) + (1ll << (kLow - 1))) >> kLow);
+    }
 };
 
 constexpr int kE = 32;       // the diagonal blocks, and the columns of a panel
@@ -153,7 +151,7 @@ constexpr int kPL = kE + 2;  // pairs from row to row of a panel in shared memor
                              // 16-byte words (16 consecutive rows fall in distinct banks)
 constexpr int kBlk = kE * kPL;
 template <int T>
-constexpr int kBlocks = T == 64 ? 5 : 2;
+constexpr int kBlocks = T == 64 ? 3 : 1;
 
 // acc(i, j) += sum_{m < 32} A[ty + 16 i][m] B[tx + 16 j][m], thread (ty, tx) =
 // (tid / 16, tid % 16); kLower: j <= i only; kRows: A and B are scaled rows.
@@ -189,192 +187,192 @@ __device__ __forceinline__ void mac(const int2* A, const int2* B, Acc<RA, RB>& a
 // other's products fill the integer pipe.
 template <int T>
 struct Smem {
-    // the sums' operand panels; then buf[0], buf[1]: C and L of a panel, or the
-    // FP64 diagonal tile; from buf[2] on: the diagonal tile's blocks
+    // the sums' operand panels; then buf[0]: C of a panel, buf[1]: L of a panel,
+    // from buf[2] on: the diagonal tile's blocks
     __align__(16) int2 buf[4][T * kPL];
-    __align__(16) int2 extra[T == 64 ? 2 : 1][T == 64 ? kBlk : 2];
-    double lraw[kE * kEL];  // the elimination's columns a_rc
-    double x[kE * kEL];     // L^-1 of the diagonal block
-    double row[2][kE];      // the published row
-    double pinv[2];
-    double piv[kE], rs[kE];  // d_c, d_c^-1/2
-    int shift[T];
-    __device__ __forceinline__ int2* blk(int i) { return i < 4 ? buf[2] + i * kBlk : extra[0]; }
-    __device__ __forceinline__ double* c() { return reinterpret_cast<double*>(buf[0]); }
+    __align__(16) int4 piv[T];
+    float part[kFxThreads];
+    // (row-major blocks, stride kPL: L_21; by columns, stride kE: L_11, L_22)
+    __device__ __forceinline__ int2* blk(int i) { return buf[2] + i * kBlk; }
+    // the columns of the L that substitute() works on
+    __align__(16) int2 cols[T * kE];
+    __device__ __forceinline__ ll* c() { return reinterpret_cast<ll*>(buf[0]); }
 };
-static_assert(sizeof(double) * 64 * 65 <= sizeof(int2) * 2 * 64 * kPL, "the diagonal tile fits two panels");
+static_assert(sizeof(ll) * 64 * kEL <= sizeof(int2) * 64 * kPL, "C of a panel fits");
 
-// 1 / d: the hardware's approximation and one step of Halley's iteration
-// y (1 + e + e^2), e = 1 - d y, which cubes its error.
-__device__ __forceinline__ double reciprocal(double d) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+// Reciprocal square root of a pivot: y 2^-61 2^((s - 3) / 2) for some s; as
+// int4 (y low, y high, the shift of a product with it, -).
+struct Pivot {
+    ll y;
+    int sh;
+};
+__device__ __forceinline__ int4 pack(const Pivot& p) { return make_int4((int)p.y, (int)(p.y >> 32), p.sh, 0); }
+__device__ __forceinline__ Pivot unpack(const int4& v) { return {(ll)(unsigned)v.x | (ll)v.y << 32, v.z}; }
+
+// 1 / sqrt(d 2^-kFrac), d > 0: v = d 2^s 2^-63 in [1/4, 1), the hardware's
+// approximation y0 of v^-1/2 and one step of the third-order iteration
+// y0 (1 + h / 2 + 3 h^2 / 8), h = 1 - v y0^2 (the series of (1 - h)^-1/2; h is
+// about 2^-21, so its error is below 2^-62).
+__device__ __forceinline__ Pivot rsqrt_pivot(ll d) {
+    int s = __clzll(d) - 1;
+    s -= (s & 1) ^ 1;  // odd: d 2^-60 = v 2^(3 - s) is then v times a power of four
+    const unsigned long long m = (unsigned long long)d << s;
+    const float v = (float)(unsigned)(m >> 32) * 0x1p-31f;
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(v));
+    const unsigned y0 = (unsigned)(yf * 0x1p30f);
+    const ll h = (1ll << 59) - (ll)__umul64hi(m, (unsigned long long)y0 * y0);  // 2^-59 steps
+    const int hh = (int)(h >> 10);
+    const ll e = (h >> 1) + ((3 * ((ll)hh * hh)) >> 42);
+    const ll y1 = (ll)y0 << 31;
+    return {y1 + (__mul64hi(y1, e << 24) >> 19), 61 - ((s - 3) >> 1)};
 }
 
-// Factors the 32 x 32 block C (row stride cl, lower triangle read, kb valid
-// rows) by elimination on [C | I] in place: at step c column c, with its
-// pivot's reciprocal, is published, every row r > c takes a_rc / d_c times
-// row c (by symmetry column c) away from its part left of the diagonal, and
-// column c, done, becomes column c of the right half. It ends with E = L'^-1,
-// C = L' D L'^T, so L^-1 = D^-1/2 E (to x) and L_rc = a_rc d_c^-1/2 (a_rc in
-// lraw, d_c^-1/2 in rs). Row c is taken from column c, not from a copy above
-// the diagonal: two copies drift apart by rounding, which a small pivot would
-// magnify. Thread t owns row t / 8 and columns 8 m + t % 8 <= row. A step is
-// one barrier and six FP64 instructions deep, and those hold the FP64 pipe
-// (each 64 cycles a warp). Returns 0 when a pivot fails its test (uniform).
-template <int T>
-__device__ __noinline__ int eliminate(Smem<T>& sm, const double* C, int cl, int kb, double eps) {
-    const int t = threadIdx.x, r = t >> 3, q = t & 7, grp = t & 31 & ~7;
-    const int mtop = (r | 3) >> 3;  // the warp's last column group
-    double w[4];
+// a times the pivot's reciprocal square root, to nearest, from limbs of 31
+// bits; bad: far above 1 (the row's squares are checked too).
+__device__ __forceinline__ ll scale_by(ll a, const Pivot& p, bool mine, int& bad) {
+    constexpr int kMask = 0x7fffffff;
+    const int a1 = (int)(a >> 31), a0 = (int)(a & kMask), y1 = (int)(p.y >> 31), y0 = (int)(p.y & kMask);
+    const ll top = (ll)a1 * y1;
+    const ll t = (ll)a1 * y0 + (ll)a0 * y1 + ((ll)a0 * y0 >> 31);
+    if (mine && (llabs(top) >> (p.sh - 1)) != 0) bad = 1;
+    return (top << (62 - p.sh)) + (t >> (p.sh - 31)) + ((t >> (p.sh - 32)) & 1);
+}
+
+// sq + (l 2^-kFrac)^2.
+__device__ __forceinline__ float add_square(float sq, ll l) {
+    const float f = (float)(int)(l >> 32) * (1.f / (1 << (kFrac - 32)));
+    return fmaf(f, f, sq);
+}
+
+// The sequential parts, a column at a time. Lane = row, and the columns of a
+// block are dealt to the NW warps of its rows: the warp that owns column c
+// finishes it (a reciprocal square root, a 64-bit product: some 60 integer
+// instructions, run by that warp alone), one barrier, and every warp takes it
+// off its own later columns. Sums are kept whole until their column is due.
+// (The inner loop stays a loop: a step's code runs once a block, and unrolled
+// 32 times it does not fit the instruction cache. Threads of one row sharing
+// its columns, with shuffles, took twice the time: every lane then runs the
+// owner's instructions.)
+//
+// Lt: the diagonal block's L by columns (row j of column c at c kE + j); part:
+// a float per thread.
+
+// Every row's squares, summed over the NW warps of its group, are within
+// their bound (uniform over the row's lanes of each group's first warp).
+template <int NW>
+__device__ __forceinline__ void check_rows(float sq, float* part, int& bad) {
+    part[threadIdx.x] = sq;
+    __syncthreads();
+    if ((threadIdx.x >> 5) % NW == 0) {
+        float v = 0.f;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const int j = 8 * m + q;
-        w[m] = j <= r ? C[r * cl + j] : 0.0;
+        for (int w = 0; w < NW; ++w) v += part[threadIdx.x + 32 * w];
+        if (!(v <= kMaxRow)) bad = 1;
     }
-    int fail = 0;
+}
+
+// Factors the 32 x 32 block C = L L^T (64-bit, row stride kEL, lower triangle
+// read): Lt (zeros above the diagonal) and piv; a pivot of the block's kb rows
+// must exceed eps in its row's scale. Returns 0 when one fails (uniform).
+__device__ __noinline__ int factor_block(const ll* C, int2* Lt, int4* piv, float* part, int kb, const Fx& d, int k0,
+                                         double eps) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ll a[4];
+    Acc<1, 4> acc;
+    acc.zero();
 #pragma unroll
-    for (int c = 0; c < kE; ++c) {
-        const int mc = c >> 3, qc = c & 7;
-        double* row = sm.row[c & 1];
-        const double arc = __shfl_sync(0xffffffffu, w[mc], grp | qc);
-        if (r == c) {
-            if (q == qc) {
-                const double d = w[mc];
-                if (c < kb && !(d > eps)) fail = 1;
-                sm.piv[c] = d;
-                sm.pinv[c & 1] = reciprocal(d);
+    for (int m = 0; m < 4; ++m) a[m] = 8 * m + warp <= lane ? C[lane * kEL + 8 * m + warp] : 0;
+    int bad = 0;
+    float sq = 0.f;
+    ll limit = 0;  // of row lane's pivot
+    if (lane < kb) {
+        int none = 0;
+        limit = max(quantize(eps, kFrac - 2 * d.e[k0 + lane], none), 0ll);
+    }
+    auto take = [&](int m, int c) {
+        const int2 l = Lt[c * kE + lane], u = Lt[c * kE + 8 * m + warp];
+        acc.add(0, m, l.x, l.y, u.x, u.y);
+    };
+#pragma unroll
+    for (int mc = 0; mc < 4; ++mc) {
+#pragma unroll 1
+        for (int qc = 0; qc < 8; ++qc) {
+            const int c = 8 * mc + qc;
+            if (warp == qc) {
+                if (c > 0) take(mc, c - 1);  // the column before, to this one alone
+                const ll v = a[mc] - acc.value(0, mc);
+                if (lane == c && !(v > limit)) bad = 1;
+                const Pivot p = rsqrt_pivot(max(__shfl_sync(0xffffffffu, v, c), 1ll));
+                ll l = scale_by(v, p, lane >= c, bad);
+                if (lane < c) l = 0;
+                Lt[c * kE + lane] = split(l);
+                if (lane == 0) piv[c] = pack(p);
+                sq = add_square(sq, l);
             }
+            if (c > 0) {  // while the owner works, and to its other columns when it is done
 #pragma unroll
-            for (int m = 0; m <= mc; ++m)
-                if (8 * m + q < c) row[8 * m + q] = w[m];
-        } else if (r > c && q == qc) {
-            row[r] = arc;
-            sm.lraw[r * kEL + c] = arc;
-        }
-        __syncthreads();
-        if (r > c) {
-            const double coef = arc * sm.pinv[c & 1];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int m = (k + ((c + 1) >> 3)) & 3;  // the next pivot's column first
-                if (m > mtop) continue;
-                if (m == mc && q == qc) w[m] = -coef;
-                else w[m] = fma(-coef, row[8 * m + q], w[m]);
+                for (int m = mc; m < 4; ++m)
+                    if (m > mc || warp > qc) take(m, c - 1);
             }
+            __syncthreads();
         }
+        if (mc == 1) acc.carry_lo();
     }
-    if (__syncthreads_or(fail)) return 0;
-    if (t < kE) sm.rs[t] = rsqrt(sm.piv[t]);
-    __syncthreads();
-    const double rr = sm.rs[r];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const int j = 8 * m + q;
-        sm.x[r * kEL + j] = j < r ? w[m] * rr : (j == r ? rr : 0.0);
-    }
-    __syncthreads();
-    return 1;
+    check_rows<8>(sq, part, bad);
+    return __syncthreads_or(bad) == 0;
 }
 
-// The diagonal block's L (zeros above the diagonal) into F. k0: its first row.
-template <int T>
-__device__ void store_block(const Fx& d, const Smem<T>& sm, int k0) {
-    const int kb = min(kE, d.n - k0);
+// L = C L_b^-T for 8 / NW groups of 32 rows: the warp's rows are lane of its
+// group, its columns NW m + its number in the group. C: row stride kEL; Lt,
+// piv: the diagonal block; out: L's rows (stride kPL), colbuf: its columns (32
+// pairs a group and column); l: the thread's entries. bad: an entry or a row's
+// squares leave their bound.
+template <int NW>
+__device__ __forceinline__ void substitute(const ll* C, const int2* Lt, const int4* piv, int2* out, int2* colbuf,
+                                           float* part, ll (&l)[kE / NW], int& bad) {
+    constexpr int CN = kE / NW;
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % NW, group = (threadIdx.x >> 5) / NW;
+    const int r = 32 * group + lane;
+    int2* mine = colbuf + group * kE * kE + lane;
+    ll a[CN];
+    Acc<1, CN> acc;
+    acc.zero();
 #pragma unroll
-    for (int m = 0; m < kE * kE / kFxThreads; ++m) {
-        const int el = threadIdx.x + m * kFxThreads, r = el >> 5, c = el & 31;
-        if (r < kb && c < kb)
-            d.F[(int64_t)(k0 + r) * d.n + k0 + c] =
-                c < r ? sm.lraw[r * kEL + c] * sm.rs[c] : (c == r ? sm.piv[r] * sm.rs[r] : 0.0);
+    for (int m = 0; m < CN; ++m) a[m] = C[r * kEL + NW * m + warp];
+    float sq = 0.f;
+    auto take = [&](int m, int c) {
+        const int2 p = mine[c * kE], u = Lt[c * kE + NW * m + warp];
+        acc.add(0, m, p.x, p.y, u.x, u.y);
+    };
+#pragma unroll
+    for (int mc = 0; mc < CN; ++mc) {
+#pragma unroll 1
+        for (int qc = 0; qc < NW; ++qc) {
+            const int c = NW * mc + qc;
+            if (warp == qc) {
+                if (c > 0) take(mc, c - 1);
+                const ll v = scale_by(a[mc] - acc.value(0, mc), unpack(piv[c]), true, bad);
+                const int2 p = split(v);
+                mine[c * kE] = p;
+                out[r * kPL + c] = p;
+                l[mc] = v;
+                sq = add_square(sq, v);
+            }
+            if (c > 0) {
+#pragma unroll
+                for (int m = mc; m < CN; ++m)
+                    if (m > mc || warp > qc) take(m, c - 1);
+            }
+            __syncthreads();
+        }
+        if (mc == CN / 2 - 1) acc.carry_lo();
     }
+    check_rows<NW>(sq, part, bad);
 }
 
-// Scales the inverse's rows: row c of X 2^{e_m} (column m) is below 2^F, kept
-// as X 2^{e_m - F - 3}, so that a product of 32 entries of C with it cannot
-// overflow; the product times 2^{F + 3} is the scaled L, shift_out[c] takes
-// its value() to kFrac. Lb: the block's L, scaled.
-template <int T>
-__device__ void scale_blocks(const Fx& d, Smem<T>& sm, int k0, int2* X, int2* Lb, int* shift_out, int& bad) {
-    const int t = threadIdx.x, r = t >> 3, q = t & 7;
-    const int er = d.e[k0 + r];
-    double v[4];
-    int em[4], top = -8192;
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const int j = 8 * m + q;
-        v[m] = sm.x[r * kEL + j];
-        em[m] = d.e[k0 + j];
-        top = max(top, exponent(v[m]) + em[m]);
-    }
-#pragma unroll
-    for (int off = 1; off < 8; off <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, off));
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const int j = 8 * m + q;
-        X[r * kPL + j] = split(quantize(v[m], kFrac - 3 + em[m] - top, bad));
-        const double l = j < r ? sm.lraw[r * kEL + j] * sm.rs[j] : (j == r ? sm.piv[r] * sm.rs[r] : 0.0);
-        Lb[r * kPL + j] = split(quantize(l, kFrac - er, bad));
-    }
-    if (q == 0) shift_out[r] = top + 3 + kFrac - kAccFrac;
-}
-
-// The rows ty + 16 a, columns tx + 16 b (b < 2) of L = C L_kk^-T from the
-// scaled C in c: the product with the inverse X, then its correction with the
-// residual against Lb = L_kk. bufC, bufL: panels of 16 RA rows; L stays in
-// bufL (visible after the caller's barrier), bad is set where a row of L
-// leaves its bound.
-template <int RA>
-__device__ __forceinline__ void solve_panel(const ll (&c)[RA][2], ll (&l)[RA][2], const int2* X, const int2* Lb,
-                                            const int (&sh)[2], int2* bufC, int2* bufL, int& bad) {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    Acc<RA, 2> u;
-    auto at = [&](int a, int b) { return (ty + 16 * a) * kPL + tx + 16 * b; };
-#pragma unroll
-    for (int a = 0; a < RA; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            if (llabs(c[a][b]) > kMaxQ) bad = 1;
-            bufC[at(a, b)] = split(c[a][b]);
-        }
-    __syncthreads();
-    u.zero();
-    mac<false, false>(bufC, X, u);
-#pragma unroll
-    for (int a = 0; a < RA; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const ll v = u.value(a, b);
-            if (llabs(v) > (sh[b] > 0 ? kMaxQ >> min(sh[b], 63) : (1ll << 62))) bad = 1;
-            l[a][b] = shift(v, sh[b]);
-            bufL[at(a, b)] = split(l[a][b]);
-        }
-    __syncthreads();
-    u.zero();
-    mac<false, true>(bufL, Lb, u);
-#pragma unroll
-    for (int a = 0; a < RA; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) bufC[at(a, b)] = split(c[a][b] - u.value_q(a, b));
-    __syncthreads();
-    u.zero();
-    mac<false, false>(bufC, X, u);
-#pragma unroll
-    for (int a = 0; a < RA; ++a) {
-        float sq = 0.f;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            l[a][b] += shift(u.value(a, b), sh[b]);
-            bufL[at(a, b)] = split(l[a][b]);
-            const float f = (float)(int)(l[a][b] >> 32) * (1.f / (1 << (kFrac - 32)));
-            sq = fmaf(f, f, sq);
-        }
-#pragma unroll
-        for (int off = 1; off < 16; off <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-        if (!(sq <= kMaxRow)) bad = 1;
-    }
+__device__ __forceinline__ double to_double(const int2& p, int e) {
+    return (double)(((ll)p.y << kLow) + p.x) * pow2(e - kFrac);
 }
 
 __device__ __forceinline__ void give_up(const Fx& d) {
@@ -430,11 +428,11 @@ __device__ void publish(const Fx& d, int* f, int task) {
 
 // kRows x 32 contiguous pairs into a panel in shared memory, asynchronously.
 template <int kRows>
-__device__ __forceinline__ void load_panel(const int2* src, int2* dst) {
+__device__ __forceinline__ void load_panel(const int2* src, int2* dst, int stride = kPL) {
 #pragma unroll
     for (int k = 0; k < kRows * kE / 2 / kFxThreads; ++k) {
         const int el = threadIdx.x + k * kFxThreads, r = el >> 4, c = 2 * (el & 15);
-        cp_async16(dst + r * kPL + c, src + r * kE + c);
+        cp_async16(dst + r * stride + c, src + r * kE + c);
     }
 }
 
@@ -486,54 +484,44 @@ __device__ bool accumulate(const Fx& d, int i, int j, Smem<T>& sm, Acc<T / 16, T
     return true;
 }
 
-// The diagonal tile jb from its FP64 lower triangle in sm.c(): factor, scaled
-// blocks and L.
+__device__ __forceinline__ ll load_scaled(const Fx& d, int row, int col, int& bad) {
+    const double v = row < d.n && col < d.n ? __ldg(d.S + (int64_t)row * d.n + col) : (row == col ? 1.0 : 0.0);
+    return quantize(v, kFrac - d.e[row] - d.e[col], bad);
+}
+
+// The diagonal tile jb from its scaled lower triangle: thread (ty, tx) holds
+// c[a][b] at (ty + 16 a, tx + 16 b), b <= a.
 template <int T>
-__device__ bool finish_diag(const Fx& d, int jb, int task, Smem<T>& sm, int bad) {
-    constexpr int CL = T + 1;
+__device__ bool finish_diag(const Fx& d, int jb, int task, Smem<T>& sm, ll (&c)[T / 16][T / 16], int bad) {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int k0 = T * jb;
     const double eps = __ldcg(&d.st->eps_factor);
-    double* c = sm.c();
-    int ok = eliminate<T>(sm, c, CL, min(kE, d.n - k0), eps);
-    if (!ok) bad = 1;
-    ll l21[2][2];
-    if constexpr (T == 32) {
-        if (ok) scale_blocks<T>(d, sm, k0, sm.blk(0), sm.blk(1), sm.shift, bad);
-    } else if (ok) {
-        scale_blocks<T>(d, sm, k0, sm.blk(0), sm.blk(2), sm.shift, bad);
-        // L_21 = C_21 L_11^-T, then C_22 -= L_21 L_21^T
-        ll q[2][2];
+    ll* C = sm.c();
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b <= a; ++b) C[(ty + 16 * a) * kEL + tx + 16 * b] = c[a][b];
+    __syncthreads();
+    if (!factor_block(C, sm.blk(0), sm.piv, sm.part, min(kE, d.n - k0), d, k0, eps)) bad = 1;
+    if constexpr (T == 64) {
+        // L_21 = C_21 L_11^-T, C_22 -= L_21 L_21^T
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int r = kE + ty + 16 * a, cc = tx + 16 * b;
-                q[a][b] = quantize(c[r * CL + cc], kFrac - d.e[k0 + r] - d.e[k0 + cc], bad);
-            }
+            for (int b = 0; b < 2; ++b) C[(ty + 16 * a) * kEL + tx + 16 * b] = c[2 + a][b];
         __syncthreads();
-        const int sh[2] = {sm.shift[tx], sm.shift[tx + 16]};
-        solve_panel<2>(q, l21, sm.blk(0), sm.blk(2), sh, sm.extra[1], sm.blk(1), bad);
-        store_block<T>(d, sm, k0);
+        ll l[4];
+        substitute<8>(C, sm.blk(0), sm.piv, sm.blk(1), sm.cols, sm.part, l, bad);
         __syncthreads();
         Acc<2, 2> u;
         u.zero();
-        mac<false, true>(sm.blk(1), sm.blk(1), u);
+        mac<true, true>(sm.blk(1), sm.blk(1), u);
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-            const int r = kE + ty + 16 * a;
-            const double sr = pow2(d.e[k0 + r] - kAccFrac);
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int cc = kE + tx + 16 * b;
-                if (cc <= r)
-                    c[r * CL + cc] = fma(-(double)u.value(a, b) * sr, pow2(d.e[k0 + cc]), c[r * CL + cc]);
-            }
-        }
+            for (int b = 0; b <= a; ++b) C[(ty + 16 * a) * kEL + tx + 16 * b] = c[2 + a][2 + b] - u.value(a, b);
         __syncthreads();
-        ok = eliminate<T>(sm, c + kE * CL + kE, CL, min(kE, d.n - k0 - kE), eps);
-        if (!ok) bad = 1;
-        if (ok) scale_blocks<T>(d, sm, k0 + kE, sm.blk(4), sm.blk(3), sm.shift + kE, bad);
+        if (!factor_block(C, sm.blk(2), sm.piv + kE, sm.part, min(kE, d.n - k0 - kE), d, k0 + kE, eps)) bad = 1;
     }
     if (__syncthreads_or(bad)) {
         give_up(d);
@@ -543,56 +531,32 @@ __device__ bool finish_diag(const Fx& d, int jb, int task, Smem<T>& sm, int bad)
 #pragma unroll
     for (int k = 0; k < kBlocks<T> * kE * kE / kFxThreads; ++k) {
         const int el = threadIdx.x + k * kFxThreads, bl = el >> 10, r = (el >> 5) & 31;
-        out[el] = sm.blk(bl)[r * kPL + (el & 31)];
+        out[el] = sm.blk(bl)[r * (bl == 1 ? kPL : kE) + (el & 31)];
     }
-    if (threadIdx.x < T) d.f[k0 + threadIdx.x] = sm.shift[threadIdx.x];
+    if (threadIdx.x < T) d.f[k0 + threadIdx.x] = sm.piv[threadIdx.x];
     publish(d, d.flag + tri(jb, jb), task);
-    if (k0 + T - kE < d.n) store_block<T>(d, sm, k0 + T - kE);
-    if constexpr (T == 64) {
+    // L into F, zeros above the diagonal
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-            const int row = k0 + kE + ty + 16 * a;
-            const double sr = pow2(d.e[row] - kFrac);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int col = k0 + tx + 16 * b;
-                if (row < d.n && col < d.n) d.F[(int64_t)row * d.n + col] = (double)l21[a][b] * sr;
-            }
-        }
+    for (int k = 0; k < kBlocks<T> * kE * kE / kFxThreads; ++k) {
+        const int el = threadIdx.x + k * kFxThreads, bl = el >> 10;
+        const int r = (el >> 5) & 31, cc = el & 31, at = bl == 1 ? r * kPL + cc : cc * kE + r;
+        const int row = k0 + r + (bl > 0 ? kE : 0), col = k0 + cc + (bl > 1 ? kE : 0);
+        if (row < d.n && col < d.n) d.F[(int64_t)row * d.n + col] = to_double(sm.blk(bl)[at], d.e[row]);
     }
     __syncthreads();
     return true;
 }
 
-__device__ __forceinline__ double load_s(const Fx& d, int row, int col) {
-    return row < d.n && col < d.n ? __ldg(d.S + (int64_t)row * d.n + col) : (row == col ? 1.0 : 0.0);
-}
-
-// sm.c() = S_ii - accD in FP64 (lower triangle; s: the thread's entries of S_ii).
+// c = S_ii - accD, scaled (lower triangle).
 template <int T>
-__device__ void diag_difference(const Fx& d, int i, Smem<T>& sm, const Acc<T / 16, T / 16>& accD,
-                                const double (&s)[T / 16][T / 16]) {
-    constexpr int R = T / 16;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double* out = sm.c();
-#pragma unroll
-    for (int a = 0; a < R; ++a) {
-        const double sr = pow2(d.e[T * i + ty + 16 * a] - kAccFrac);
-#pragma unroll
-        for (int b = 0; b <= a; ++b) {
-            const int r = ty + 16 * a, c = tx + 16 * b;
-            out[r * (T + 1) + c] = fma(-(double)accD.value(a, b) * sr, pow2(d.e[T * i + c]), s[a][b]);
-        }
-    }
-}
-
-template <int T>
-__device__ __forceinline__ void load_diag_s(const Fx& d, int i, double (&s)[T / 16][T / 16]) {
+__device__ __forceinline__ void diag_difference(const Fx& d, int i, const Acc<T / 16, T / 16>& accD,
+                                                ll (&c)[T / 16][T / 16], int& bad) {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
     for (int a = 0; a < T / 16; ++a)
 #pragma unroll
-        for (int b = 0; b <= a; ++b) s[a][b] = load_s(d, T * i + ty + 16 * a, T * i + tx + 16 * b);
+        for (int b = 0; b <= a; ++b)
+            c[a][b] = load_scaled(d, T * i + ty + 16 * a, T * i + tx + 16 * b, bad) - accD.value(a, b);
 }
 
 // Tile (i, j), i > j; with kD (T = 32) also the diagonal tile i = j + 1, whose
@@ -600,102 +564,93 @@ __device__ __forceinline__ void load_diag_s(const Fx& d, int i, double (&s)[T / 
 // a column.
 template <int T, bool kD>
 __device__ bool task_tile(const Fx& d, int i, int j, int task, Smem<T>& sm) {
-    constexpr int R = T / 16, H = T / kE;
+    constexpr int R = T / 16, H = T / kE, NW = kFxThreads / T, CN = kE / NW;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int r = (threadIdx.x >> 5) / NW * 32 + (threadIdx.x & 31), q = (threadIdx.x >> 5) % NW;  // as substitute()
     int bad = 0;
-    ll cq[H][R][2];  // the tile's entries of S, scaled; then of C; then of L
+    ll cq[R][R];  // the tile's entries of S, scaled; then of C
     auto load = [&] {
 #pragma unroll
-        for (int h = 0; h < H; ++h)
+        for (int a = 0; a < R; ++a)
 #pragma unroll
-            for (int a = 0; a < R; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const int row = T * i + ty + 16 * a, col = T * j + kE * h + tx + 16 * b;
-                    cq[h][a][b] = quantize(load_s(d, row, col), kFrac - d.e[row] - d.e[col], bad);
-                }
+            for (int b = 0; b < R; ++b) cq[a][b] = load_scaled(d, T * i + ty + 16 * a, T * j + tx + 16 * b, bad);
     };
     if constexpr (T == 32) load();  // before anything is waited for (T = 64: after the sums, for their registers)
+    Acc<R, R> accD;
+    if (kD) accD.zero();
     {
-        Acc<R, R> accL, accD;
+        Acc<R, R> accL;
         accL.zero();
-        if (kD) accD.zero();
         if (!accumulate<T, true, kD>(d, i, j, sm, accL, accD, bad)) return false;
         if constexpr (T == 64) load();
 #pragma unroll
-        for (int h = 0; h < H; ++h)
+        for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b < R; ++b) cq[a][b] -= accL.value(a, b);
+    }
+    if (!wait_flags(d, d.flag + tri(j, j), d.flag + tri(j, j))) return false;
+#pragma unroll
+    for (int bl = 0; bl < kBlocks<T>; ++bl)
+        load_panel<kE>(d.G + ((int64_t)j * kBlocks<T> + bl) * kE * kE, sm.blk(bl), bl == 1 ? kPL : kE);
+    if (threadIdx.x < T) cp_async16(sm.piv + threadIdx.x, d.f + T * j + threadIdx.x);
+    cp_async_commit();
+    ll* C = sm.c();
+    ll l[H][CN];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+        if (h > 0) {  // C_2 -= L_1 L_21^T
+            Acc<R, 2> u;
+            u.zero();
+            mac<false, true>(sm.buf[1], sm.blk(1), u);
 #pragma unroll
             for (int a = 0; a < R; ++a)
 #pragma unroll
-                for (int b = 0; b < 2; ++b) cq[h][a][b] -= accL.value_q(a, 2 * h + b);
-        if (!wait_flags(d, d.flag + tri(j, j), d.flag + tri(j, j))) return false;
-#pragma unroll
-        for (int bl = 0; bl < kBlocks<T>; ++bl)
-            load_panel<kE>(d.G + ((int64_t)j * kBlocks<T> + bl) * kE * kE, sm.blk(bl));
-        cp_async_commit();
-        int sh[H][2];
-#pragma unroll
-        for (int h = 0; h < H; ++h)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) sh[h][b] = __ldcg(d.f + T * j + kE * h + tx + 16 * b);
-        double s[R][R];
-        if (kD) load_diag_s<T>(d, i, s);
-        cp_async_wait<0>();
-        // (the barrier in solve_panel makes the copies visible)
-#pragma unroll
-        for (int h = 0; h < H; ++h) {
-            if (h > 0) {  // C_2 -= L_1 L_21^T
-                Acc<R, 2> u;
-                u.zero();
-                mac<false, true>(sm.buf[1], sm.blk(1), u);
-#pragma unroll
-                for (int a = 0; a < R; ++a)
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) cq[h][a][b] -= u.value_q(a, b);
-                __syncthreads();
-            }
-            ll l[R][2];
-            solve_panel<R>(cq[h], l, sm.blk(h == 0 ? 0 : 4), sm.blk(T == 32 ? 1 : 2 + h), sh[h], sm.buf[0], sm.buf[1], bad);
-#pragma unroll
-            for (int a = 0; a < R; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    cq[h][a][b] = l[a][b];
-                    d.Q[tri(i, j) * T * T + (h * T + ty + 16 * a) * kE + tx + 16 * b] = split(l[a][b]);
-                }
-            if (h + 1 < H) __syncthreads();
+                for (int b = 0; b < 2; ++b) cq[a][2 * h + b] -= u.value(a, b);
+            // (C's and L's buffers are free: the barrier before h = 1, and the one below)
         }
-        if (__syncthreads_or(bad)) {
-            give_up(d);
-            return false;
-        }
-        publish(d, d.flag + tri(i, j), task);
-        if constexpr (kD) {
-            mac<true, true>(sm.buf[1], sm.buf[1], accD);
-            if (tx == ty) {
 #pragma unroll
-                for (int a = 0; a < R; ++a)
-                    if (accD.hi[a][a] > kMaxDiag) bad = 1;
-            }
-            diag_difference<T>(d, i, sm, accD, s);
-            __syncthreads();
+        for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) C[(ty + 16 * a) * kEL + tx + 16 * b] = cq[a][2 * h + b];
+        if (h == 0) cp_async_wait<0>();
+        __syncthreads();
+        substitute<NW>(C, sm.blk(2 * h), sm.piv + kE * h, sm.buf[1], sm.cols, sm.part, l[h], bad);
+        __syncthreads();
+        int2* Qh = d.Q + tri(i, j) * T * T + h * T * kE;
+#pragma unroll
+        for (int k = 0; k < T * kE / kFxThreads; ++k) {
+            const int el = threadIdx.x + k * kFxThreads;
+            Qh[el] = sm.buf[1][(el >> 5) * kPL + (el & 31)];
         }
     }
+    if (__syncthreads_or(bad)) {
+        give_up(d);
+        return false;
+    }
+    publish(d, d.flag + tri(i, j), task);
     if constexpr (kD) {
-        if (!finish_diag<T>(d, i, task, sm, bad)) return false;
-    }
+        mac<true, true>(sm.buf[1], sm.buf[1], accD);
+        if (tx == ty) {
 #pragma unroll
-    for (int h = 0; h < H; ++h)
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-            const int row = T * i + ty + 16 * a;
-            const double sr = pow2(d.e[row] - kFrac);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int col = T * j + kE * h + tx + 16 * b;
-                if (row < d.n && col < d.n) d.F[(int64_t)row * d.n + col] = (double)cq[h][a][b] * sr;
-            }
+            for (int a = 0; a < R; ++a)
+                if (accD.hi[a][a] > kMaxDiag) bad = 1;
         }
+        ll c[R][R];
+        diag_difference<T>(d, i, accD, c, bad);
+        __syncthreads();
+        if (!finish_diag<T>(d, i, task, sm, c, bad)) return false;
+    }
+    const int row = T * i + r;
+    if (row < d.n) {
+        const double sr = pow2(d.e[row] - kFrac);
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+#pragma unroll
+            for (int m = 0; m < CN; ++m) {
+                const int col = T * j + kE * h + NW * m + q;
+                if (col < d.n) d.F[(int64_t)row * d.n + col] = (double)l[h][m] * sr;
+            }
+    }
     __syncthreads();
     return true;
 }
@@ -704,16 +659,14 @@ __device__ bool task_tile(const Fx& d, int i, int j, int task, Smem<T>& sm) {
 template <int T>
 __device__ bool task_diag(const Fx& d, int j, int task, Smem<T>& sm) {
     int bad = 0;
+    ll c[T / 16][T / 16];
     {
         Acc<T / 16, T / 16> none, accD;
         accD.zero();
         if (!accumulate<T, false, true>(d, j, j, sm, none, accD, bad)) return false;
-        double s[T / 16][T / 16];
-        load_diag_s<T>(d, j, s);
-        diag_difference<T>(d, j, sm, accD, s);
+        diag_difference<T>(d, j, accD, c, bad);
     }
-    __syncthreads();
-    return finish_diag<T>(d, j, task, sm, bad);
+    return finish_diag<T>(d, j, task, sm, c, bad);
 }
 
 template <int T>
@@ -821,7 +774,7 @@ cudaError_t launch_chol_fx(int n, const double* S, double* F, void* work, LmStat
     d.G = reinterpret_cast<int2*>(w + l.g);
     int* e = reinterpret_cast<int*>(w + l.e);
     d.e = e;
-    d.f = reinterpret_cast<int*>(w + l.f);
+    d.f = reinterpret_cast<int4*>(w + l.f);
     d.flag = reinterpret_cast<int*>(w + l.flag);
     d.abort = d.flag + l.tiles;
     d.st = st;

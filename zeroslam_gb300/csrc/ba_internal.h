@@ -384,13 +384,13 @@ cudaError_t launch_trisolve(int n, const double* F, const double* b, double* x, 
                             cudaStream_t s);
 
 // ---- FP64 factor (ba_chol_fx.cu) ----
-// The tile edge: up to kFxSmallN the chain of diagonal tiles bounds the launch
-// and small tiles shorten it; beyond, its products do, and larger tiles read
-// and wait less per product.
-constexpr int kFxSmallN = 1536;
-struct FxLayout {  // the workspace: tiles and diagonal blocks (int2), row scales, shifts, flags
+// The tile edge. Small tiles shorten the chain of diagonal tiles, large ones
+// read and wait less per product: 32 against 64 at n = 1800 / 3000 / 4500 /
+// 6000: 1.56 / 4.15 / 11.5 / 26.5 against 2.72 / 5.10 / 11.6 / 23.6 ms.
+constexpr int kFxSmallN = 4608;
+struct FxLayout {  // the workspace: tiles and diagonal blocks (int2), pivots (int4), row scales, flags
     int T, N, tiles;
-    size_t g, e, f, flag, bytes;
+    size_t g, f, e, flag, bytes;
 };
 constexpr FxLayout fx_layout(int n) {
     FxLayout l{};
@@ -398,9 +398,9 @@ constexpr FxLayout fx_layout(int n) {
     l.N = (n + l.T - 1) / l.T;
     l.tiles = l.N * (l.N + 1) / 2;
     l.g = sizeof(int2) * (size_t)l.tiles * l.T * l.T;
-    l.e = l.g + sizeof(int2) * (size_t)l.N * (l.T == 64 ? 5 : 2) * 1024;
-    l.f = l.e + sizeof(int) * (size_t)l.N * l.T;
-    l.flag = l.f + sizeof(int) * (size_t)l.N * l.T;
+    l.f = l.g + sizeof(int2) * (size_t)l.N * (l.T == 64 ? 3 : 1) * 1024;
+    l.e = l.f + sizeof(int4) * (size_t)l.N * l.T;
+    l.flag = l.e + sizeof(int) * (size_t)l.N * l.T;
     l.bytes = l.flag + sizeof(int) * ((size_t)l.tiles + 1);
     return l;
 }
