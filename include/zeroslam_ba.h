@@ -263,7 +263,9 @@ int zs_ba_get_history(zs_ba_handle* h, zs_ba_attempt* out, int32_t capacity, int
  * (fx, fy, cx, cy) and adjoint_state [6K+3L], the solution v of H v = a.
  * H is the exact Hessian of the cost in local coordinates (Gauss-Newton term
  * plus residual curvature); H v = a is solved by conjugate gradients
- * preconditioned with the solver's Schur / reduced-Cholesky factorisation.
+ * preconditioned with a Schur / reduced-Cholesky factorisation, of H itself
+ * where it is positive definite (two or three iterations), else of its
+ * Gauss-Newton part.
  * With a = the gradient vector b of zs_ba_linear_step, v is the exact Newton
  * step. FP64 handles and ZS_LOSS_NONE only (ZS_ERR_UNSUPPORTED otherwise).
  * No counterpart in the reference. */

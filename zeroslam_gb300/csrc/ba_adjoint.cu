@@ -12,12 +12,14 @@
 // P the camera-frame point, A = dP/dx = [-[P]x | I | R], Pi_k the Hessian of
 // the projection (source/camera.hpp:91-142) and d2 P the second-order terms of
 // exp(d) (P + R dl): 1/2 w x (w x P) + 1/2 w x u + w x (R dl).
-// H v = a is solved by conjugate gradients preconditioned with the solver's
-// lightly damped Gauss-Newton factorisation (Schur complement + reduced
-// Cholesky): the factor is reused, only exact-Hessian products are new. H is
-// symmetric positive definite at an isolated minimum; CG also converges where
-// the curvature term is not small against the Gauss-Newton block (landmarks
-// seen with little parallax), where a plain preconditioned iteration stalls.
+// H v = a is solved by conjugate gradients preconditioned with a lightly damped
+// factorisation (Schur complement + reduced Cholesky). H has the blocks of the
+// Gauss-Newton matrix, one for each (pose, landmark) pair and on the diagonal,
+// and is positive definite at an isolated minimum: the factorisation is then
+// of H itself, and two or three iterations leave its rounding behind
+// (preconditioned with the Gauss-Newton matrix the same scene took 48). Where
+// H is not positive definite (or a landmark's block is singular: seen once, or
+// not at all) the preconditioner is the Gauss-Newton factorisation.
 // There is no counterpart in the reference; the gradient is checked against
 // central finite differences of whole solves.
 #include "ba_internal.h"
@@ -104,6 +106,66 @@ __global__ void __launch_bounds__(kThreads) k_adj_prep(DevProblem P, double* __r
             out[idx++] = -(aca + g);
         }
     }
+}
+
+// The 9 x 9 block H_o = J^T Omega J + Q of each observation, in the places and
+// layouts of k_linearize<double>: the 6 x 3 pose-landmark part and the pose's
+// 21 entries at its pose-major position, the landmark's 6 entries (fixed
+// vertices zero; no gradient).
+__global__ void __launch_bounds__(kThreads) k_adj_blocks(DevProblem P, const double* __restrict__ rec,
+                                                         double* __restrict__ hpl, double* __restrict__ lm_part,
+                                                         double* __restrict__ pose_part) {
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= P.M) return;
+    const int64_t o = P.pose_obs[q];
+    const bool pf = P.pose_fixed[P.obs_pose[o]] != 0, lf = P.lm_fixed[P.obs_lm[o]] != 0;
+    const double2* r2 = reinterpret_cast<const double2*>(rec + o * kAdjRec);
+    double v[64];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        const double2 t = __ldg(r2 + i);
+        v[2 * i] = t.x;
+        v[2 * i + 1] = t.y;
+    }
+    double W[4] = {1.0, 0.0, 0.0, 1.0};
+    if (P.obs_info)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) W[i] = P.obs_info[4 * o + i];
+    double A0[9], A1[9];  // (J^T Omega) columns
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        A0[i] = v[i] * W[0] + v[9 + i] * W[2];
+        A1[i] = v[i] * W[1] + v[9 + i] * W[3];
+    }
+    double* ph = pose_part + q * 28;
+    double* lh = lm_part + o * 12;
+    int idx = 18, up = 0, ul = 0;
+#pragma unroll
+    for (int a = 0; a < 9; ++a)
+#pragma unroll
+        for (int b = a; b < 9; ++b) {
+            const double h = A0[a] * v[b] + A1[a] * v[9 + b] + v[idx++];
+            if (b < 6) ph[up++] = pf ? 0.0 : h;
+            else if (a < 6) hpl[q * 18 + a * 3 + (b - 6)] = pf || lf ? 0.0 : h;
+            else lh[ul++] = lf ? 0.0 : h;
+        }
+#pragma unroll
+    for (int i = 21; i < 28; ++i) ph[i] = 0.0;
+#pragma unroll
+    for (int i = 6; i < 12; ++i) lh[i] = 0.0;
+}
+
+__global__ void __launch_bounds__(kThreads) k_adj_check_lm(DevProblem P, const double* __restrict__ hll, LmState* st) {
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= P.L || P.lm_fixed[l]) return;
+    double a[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) a[i] = hll[(int64_t)l * 9 + i];
+    a[0] += st->lambda; a[4] += st->lambda; a[8] += st->lambda;
+    const double d2 = a[0] * a[4] - a[1] * a[3];
+    const double det = a[0] * (a[4] * a[8] - a[7] * a[5]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);
+    const double m = fmax(a[0], fmax(a[4], a[8]));
+    if (!(a[0] > 0.0 && d2 > 0.0 && det > 1e-12 * m * m * m)) st->solve_ok = 0;
 }
 
 // y_o = (J^T Omega J + Q) v_o for v = (v_pose, v_landmark); the 9 values go
@@ -400,6 +462,20 @@ void launch_adj_apply_inverse(int n, const double* Xi, const double* XiT, const 
 void launch_adj_prep(const DevProblem& P, double* rec, cudaStream_t s) {
     if (P.M > 0) {
         k_adj_prep<<<grid_for(P.M), kThreads, 0, s>>>(P, rec);
+        note_launch();
+    }
+}
+
+void launch_adj_blocks(const DevProblem& P, const double* rec, DevWork& W, cudaStream_t s) {
+    if (P.M > 0) {
+        k_adj_blocks<<<grid_for(P.M), kThreads, 0, s>>>(P, rec, (double*)W.hpl, (double*)W.lm_part, (double*)W.pose_part);
+        note_launch();
+    }
+}
+
+void launch_adj_check_lm(const DevProblem& P, const DevWork& W, LmState* st, cudaStream_t s) {
+    if (P.L > 0) {
+        k_adj_check_lm<<<grid_for(P.L), kThreads, 0, s>>>(P, W.hll, st);
         note_launch();
     }
 }

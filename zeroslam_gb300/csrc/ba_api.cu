@@ -1689,7 +1689,6 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
             h->adj_rec = dalloc<double>((size_t)std::max<int64_t>(P.M, 1) * kAdjRecord, h->owned);
             h->adj_part = dalloc<double>((size_t)std::max<int64_t>(P.M, 1) * 9, h->owned);
             h->adj_vec = dalloc<double>((size_t)std::max<int64_t>(N, 1) * 7, h->owned);
-            if (n > 0 && n <= kAdjInvMaxN) h->adj_inv = dalloc<double>((size_t)n * (2 * (size_t)n + 1), h->owned);
         }
         double* a = h->adj_vec;
         double* v = a + N;
@@ -1707,22 +1706,35 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
         if (N > 0) ZS_CUDA(cudaMemcpyAsync(a, ah.data(), N * sizeof(double), cudaMemcpyHostToDevice, s));
         ZS_CUDA(cudaMemsetAsync(v, 0, std::max<int64_t>(N, 1) * sizeof(double), s));
         ZS_CUDA(cudaMemsetAsync(zero, 0, std::max<int64_t>(N, 1) * sizeof(double), s));
-        // Gauss-Newton linearisation and its lightly damped factorisation:
-        // the preconditioner M = H_GN + lambda I.
-        linearize<double>(h);
+        // The preconditioner M: the lightly damped factorisation of the exact
+        // Hessian, or where that is not positive definite of the
+        // Gauss-Newton matrix. (The exact one is M = H but for the damping, so
+        // its damping is only what the fixed poses' zero rows need to pass the
+        // pivot test.)
         launch_adj_prep(P, h->adj_rec, s);
-        launch_cost(P, W, h->st, false, s);
-        launch_init_lambda(P, W, h->st, h->opt.tau, h->opt.diagonal_clamp, s);
-        read_state(h);
-        LmState init{};
-        init.lambda = 1e-9 * std::max(h->st_host->max_diag, 1e-300);
-        init.nu = 2.0;
-        init.solve_ok = 1;
-        ZS_CUDA(cudaMemcpyAsync(h->st, &init, sizeof(LmState), cudaMemcpyHostToDevice, s));
-        launch_invert_w<double>(P, W, h->st, s);
-        launch_schur<double>(P, W, h->st, s);
-        ZS_CUDA(launch_chol_fx(n, W.S, (double*)W.F, W.fx, h->st, s));
-        read_state(h);
+        bool exact = true;
+        for (;; exact = false) {
+            if (exact) {
+                launch_adj_blocks(P, h->adj_rec, W, s);
+                launch_block_sums<double>(P, W, s);
+            } else {
+                linearize<double>(h);
+            }
+            launch_cost(P, W, h->st, false, s);
+            launch_init_lambda(P, W, h->st, h->opt.tau, h->opt.diagonal_clamp, s);
+            read_state(h);
+            LmState init{};
+            init.lambda = (exact ? 1e-13 : 1e-9) * std::max(h->st_host->max_diag, 1e-300);
+            init.nu = 2.0;
+            init.solve_ok = 1;
+            ZS_CUDA(cudaMemcpyAsync(h->st, &init, sizeof(LmState), cudaMemcpyHostToDevice, s));
+            if (exact) launch_adj_check_lm(P, W, h->st, s);
+            launch_invert_w<double>(P, W, h->st, s);
+            launch_schur<double>(P, W, h->st, s);
+            ZS_CUDA(launch_chol_fx(n, W.S, (double*)W.F, W.fx, h->st, s));
+            read_state(h);
+            if (!exact || h->st_host->solve_ok || h->st_host->timeout) break;
+        }
         if (!h->st_host->solve_ok) {
             status = h->st_host->timeout ? ZS_ERR_TIMEOUT : ZS_ERR_CHOLESKY;
         } else {
@@ -1736,9 +1748,13 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 return t;
             };
             // z = M^-1 x through the Schur complement and the reduced factor;
-            // up to kAdjInvMaxN the factor's inverse is formed once and each
-            // reduced solve is two triangular products
-            double* Xi = h->adj_inv;
+            // for the Gauss-Newton preconditioner's many iterations, up to
+            // kAdjInvMaxN, the factor's inverse is formed once and each reduced
+            // solve is two triangular products (14 us against 55 at n = 300;
+            // the inverse takes 570)
+            if (!exact && n > 0 && n <= kAdjInvMaxN && !h->adj_inv)
+                h->adj_inv = dalloc<double>((size_t)n * (2 * (size_t)n + 1), h->owned);
+            double* Xi = exact ? nullptr : h->adj_inv;
             double* XiT = Xi ? Xi + (size_t)n * n : nullptr;
             if (Xi) launch_adj_tri_inverse(n, (const double*)W.F, Xi, XiT, s);
             auto precondition = [&](const double* x, double* out) {
@@ -1765,9 +1781,10 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                     std::fprintf(stderr, "zs adjoint: |a| %.6e  r.Mr %.6e  |M^-1 a| %.6e\n", anorm, rz,
                                  std::sqrt(dot(z, z)));
                 // The iterations run with their scalars on the device
-                // (AdjCg): the host enqueues kAdjBatch of them at a time and
+                // (AdjCg): the host enqueues a batch of them at a time and
                 // reads the stop flag once per batch; iterations enqueued past
-                // the stop change nothing.
+                // the stop change nothing. (With the exact Hessian's
+                // factorisation two or three iterations are all there are.)
                 AdjCg c0{};
                 c0.rz = rz;
                 c0.anorm = anorm;
@@ -1777,9 +1794,9 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 ZS_CUDA(cudaMemcpyAsync(cg, &c0, sizeof(AdjCg), cudaMemcpyHostToDevice, s));
                 double* red2 = W.red + kReduceBlocks;  // the loop's partial sums
                 AdjCg ch = c0;
-                constexpr int kAdjBatch = 8;
+                const int batch = exact ? 2 : 8;
                 while (!ch.done) {
-                    for (int b = 0; b < kAdjBatch; ++b) {
+                    for (int b = 0; b < batch; ++b) {
                         launch_adj_residual(P, h->adj_rec, pv, zero, h->adj_part, W.opch_sum, q, s);  // q = -H p
                         launch_adj_dot(N, pv, q, red2, s);
                         launch_adj_cg_pap(red2, cg, s);                // alpha = rz / p.Hp

@@ -208,6 +208,10 @@ int record_cuda_error(cudaError_t e);
 // ---- kernels (ba_kernels.cu) ----
 template <typename T>
 void launch_linearize(const DevProblem& P, DevWork& W, cudaStream_t s);
+// The sums of the per-observation records that launch_linearize's first
+// kernel (or launch_adj_blocks) left: duplicates merged, H_ll, H_pp and b.
+template <typename T>
+void launch_block_sums(const DevProblem& P, DevWork& W, cudaStream_t s);
 template <typename T>
 void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
 template <typename T>
@@ -310,6 +314,12 @@ int bsolve_max_blocks_per_sm(int bucket, int threads);
 // ---- adjoint (ba_adjoint.cu) ----
 constexpr int kAdjRecord = 64;  // doubles per observation in the adjoint record
 void launch_adj_prep(const DevProblem& P, double* rec, cudaStream_t s);
+// The exact Hessian's blocks per observation, from the records, where
+// launch_linearize leaves the Gauss-Newton ones.
+void launch_adj_blocks(const DevProblem& P, const double* rec, DevWork& W, cudaStream_t s);
+// st->solve_ok = 0 unless every free landmark's H_ll + lambda I is positive
+// definite and passes the inverse's determinant test.
+void launch_adj_check_lm(const DevProblem& P, const DevWork& W, LmState* st, cudaStream_t s);
 void launch_adj_residual(const DevProblem& P, const double* rec, const double* v, const double* a, double* part,
                          double* csum, double* out, cudaStream_t s);
 // The adjoint's preconditioner with an explicit inverse of its fixed FP64

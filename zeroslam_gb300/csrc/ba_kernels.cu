@@ -1262,8 +1262,13 @@ void launch_linearize(const DevProblem& P, DevWork& W, cudaStream_t s) {
     if (P.M > 0) {
         k_linearize<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl, (T*)W.lm_part, (T*)W.pose_part, W.pose_aux,
                                                           W.jac, P.pose_win ? nullptr : W.jp_pm); note_launch();
-        if (P.has_dups) { k_merge_dups<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl); note_launch(); }
     }
+    launch_block_sums<T>(P, W, s);
+}
+
+template <typename T>
+void launch_block_sums(const DevProblem& P, DevWork& W, cudaStream_t s) {
+    if (P.M > 0 && P.has_dups) { k_merge_dups<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl); note_launch(); }
     if (P.L > 0) {
         if (sizeof(T) == 4) {
             // a thread per landmark when they fill the GPU, else warps over chunks
@@ -1385,6 +1390,7 @@ void launch_set_solve_ok(LmState* st, int v, cudaStream_t s) { k_set_solve_ok<<<
 
 template void launch_linearize<double>(const DevProblem&, DevWork&, cudaStream_t);
 template void launch_linearize<float>(const DevProblem&, DevWork&, cudaStream_t);
+template void launch_block_sums<double>(const DevProblem&, DevWork&, cudaStream_t);
 template void launch_invert_w<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_invert_w<float>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_schur<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
