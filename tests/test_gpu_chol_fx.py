@@ -48,6 +48,20 @@ def test_factor(zs_lib, n, kind):
     assert r <= 40 * (n + 2) * 2.0**-53 * np.linalg.norm(A, 2) * np.linalg.norm(x)
 
 
+@pytest.mark.parametrize("n", [1, 2, 33, 70, 4640])
+def test_pivots_of_powers_of_four(zs_lib, n):
+    """Pivots that are powers of four, the lowest of their scaled range, and
+    factors that FP64 holds: L's diagonal is the positive root."""
+    rng = np.random.default_rng(n)
+    L = np.eye(n) + np.diag(rng.choice([-0.25, 0.0, 0.25], n - 1), -1)
+    L = 2.0 ** rng.integers(-3, 4, n)[:, None] * L
+    ok, F, _ = ba.dense_cholesky_solve(L @ L.T, np.ones(n))
+    assert ok
+    # A pivot's error is a few 2^-60 of its scale and what it passes on shrinks
+    # sixteenfold from row to row: the last conversion's 2^-53 and as much again.
+    assert (np.abs(F - L) <= 2.0**-52 * np.sqrt(np.diag(L @ L.T))[:, None]).all()
+
+
 @pytest.mark.parametrize("n", [4608, 4609, 4641, 4705])
 def test_factor_large(zs_lib, n):
     """Either side of the change of tiles (n = 4608), and the 64-wide tiles' ragged ends."""

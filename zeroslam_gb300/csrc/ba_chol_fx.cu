@@ -200,7 +200,7 @@ struct Smem {
 };
 static_assert(sizeof(ll) * 64 * kEL <= sizeof(int2) * 64 * kPL, "C of a panel fits");
 
-// Reciprocal square root of a pivot: y 2^-61 2^((s - 3) / 2) for some s; as
+// Reciprocal square root of a pivot: y 2^-61 2^((s - 3) / 2) for some s, y < 2^62; as
 // int4 (y low, y high, the shift of a product with it, -).
 struct Pivot {
     ll y;
@@ -225,7 +225,8 @@ __device__ __forceinline__ Pivot rsqrt_pivot(ll d) {
     const int hh = (int)(h >> 10);
     const ll e = (h >> 1) + ((3 * ((ll)hh * hh)) >> 42);
     const ll y1 = (ll)y0 << 31;
-    return {y1 + (__mul64hi(y1, e << 24) >> 19), 61 - ((s - 3) >> 1)};
+    // (v = 1/4 ends at 2^62, which the upper of scale_by's limbs does not hold)
+    return {min(y1 + (__mul64hi(y1, e << 24) >> 19), (1ll << 62) - 1), 61 - ((s - 3) >> 1)};
 }
 
 // a times the pivot's reciprocal square root, to nearest, from limbs of 31
