@@ -1118,7 +1118,7 @@ void read_state(zs_ba_handle* h) {
 template <typename T>
 void linearize(zs_ba_handle* h) {
     PhaseScope ps(h->timer, ZS_PHASE_LINEARIZE, h->stream);
-    launch_linearize<T>(h->P, h->W, h->stream);
+    launch_linearize<T>(h->P, h->W, nullptr, h->stream);
 }
 
 // Mixed form: relative diagonal shift of the preconditioner's retry
@@ -1163,7 +1163,7 @@ void system_solve(zs_ba_handle* h) {
     }
     if constexpr (sizeof(T) == 8) {
         PhaseScope ps(h->timer, ZS_PHASE_UPDATE, s);
-        launch_backsub<T>(P, W, h->st, s);
+        launch_backsub(P, W, h->st, s);
     }
 }
 
@@ -1716,7 +1716,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
         for (;; exact = false) {
             if (exact) {
                 launch_adj_blocks(P, h->adj_rec, W, s);
-                launch_block_sums<double>(P, W, s);
+                launch_block_sums<double>(P, W, nullptr, s);
             } else {
                 linearize<double>(h);
             }
@@ -1765,7 +1765,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 } else {
                     ZS_CUDA(launch_trisolve(n, (const double*)W.F, W.bs, W.delta, W.work, h->st, s));
                 }
-                launch_backsub<double>(P, W, h->st, s);
+                launch_backsub(P, W, h->st, s);
                 launch_adj_copy(N, W.delta, out, s);
             };
             launch_adj_residual(P, h->adj_rec, v, a, h->adj_part, W.opch_sum, r, s);  // r = a, fixed entries zeroed

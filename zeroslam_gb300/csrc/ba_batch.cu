@@ -636,7 +636,7 @@ int bsolve_max_blocks_per_sm(int bucket, int threads) {
 template <typename T>
 void launch_batch_prologue(const DevProblem& P, DevWork& W, BatchDev& B, const BatchParams& prm, cudaStream_t s) {
     k_breset<<<1, 32, 0, s>>>(B.counters, B.any_active, B.rounds); note_launch();
-    launch_linearize<T>(P, W, s);  // (mixed form: also the per-pose sandwich matrices)
+    launch_linearize<T>(P, W, nullptr, s);  // (mixed form: also the per-pose sandwich matrices)
     const double* aux = sizeof(T) == 4 ? W.pose_aux : nullptr;
     if (P.nochunks > 0) { k_bcost_partial<<<(int)P.nochunks, kThreads, 0, s>>>(P, aux, W.red, B.st, B.ctl, 1); note_launch(); }
     k_bcost_finish<<<grid_for(P.nwin), kThreads, 0, s>>>(P, W.red, B.st, B.ctl, 1); note_launch();
@@ -646,7 +646,6 @@ void launch_batch_prologue(const DevProblem& P, DevWork& W, BatchDev& B, const B
 template <typename T>
 cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, const BatchParams& prm,
                                cudaStream_t s) {
-    launch_linearize<T>(P, W, s);
     if (P.L > 0) {
         k_binvert<<<grid_for(std::max(P.L, W.row_exp ? 12 * P.K : 0)), kThreads, 0, s>>>(
             P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, W.lm_exp, W.row_exp,
@@ -690,6 +689,8 @@ cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, con
     k_bcost_finish<<<grid_for(P.nwin), kThreads, 0, s>>>(P, W.red, B.st, B.ctl, 0); note_launch();
     k_bdecide<<<1, kThreads, 0, s>>>(P.nwin, B.st, B.ctl, prm, B.counters, B.any_active, B.rounds); note_launch();
     k_brollback<<<grid_for((int64_t)P.K + P.L), kThreads, 0, s>>>(P, B.ctl); note_launch();
+    // for the next round, if there is one (the first round's is the prologue's)
+    launch_linearize<T>(P, W, B.any_active, s);
     return cudaGetLastError();
 }
 

@@ -206,17 +206,17 @@ struct WinCtl {
 int record_cuda_error(cudaError_t e);
 
 // ---- kernels (ba_kernels.cu) ----
+// (go: every kernel returns at once when *go is 0; null: they run)
 template <typename T>
-void launch_linearize(const DevProblem& P, DevWork& W, cudaStream_t s);
+void launch_linearize(const DevProblem& P, DevWork& W, const int* go, cudaStream_t s);
 // The sums of the per-observation records that launch_linearize's first
 // kernel (or launch_adj_blocks) left: duplicates merged, H_ll, H_pp and b.
 template <typename T>
-void launch_block_sums(const DevProblem& P, DevWork& W, cudaStream_t s);
+void launch_block_sums(const DevProblem& P, DevWork& W, const int* go, cudaStream_t s);
 template <typename T>
 void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
 template <typename T>
 void launch_schur(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
-template <typename T>
 void launch_backsub(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
 // b_s = b_p - W b_l from the current W.b (no other Schur work).
 template <typename T>
@@ -534,10 +534,38 @@ size_t pcg_doubles(const DevProblem& P);
 // Per-pose sums of six values over each pose's observations, spread over the
 // whole GPU (a CTA per pose leaves most SMs idle at a few hundred poses) in a
 // fixed order: a warp per pose-major chunk (<= kOpChunk positions of one
-// pose, P.opch_q; lane i takes positions i, i + 32, then a butterfly) into
-// part[6 c + a], then a thread per (pose, value) adds its pose's chunks in
-// chunk order and hands the total to out(P, k, a, total). term(P, q, s) adds
-// position q's six values to s.
+// pose, P.opch_q; lane i takes positions i, i + 32, then warp_sum6) into
+// part[6 c + a], then a warp per pose adds its chunks (lane i takes chunks i,
+// i + 32, ..., then warp_sum6) and hands the totals to out(P, k, a, total).
+// term(P, q, s) adds position q's six values to s.
+//
+// The six values' sums over a warp: halves of the warp exchange three values
+// each, then quarters, and so on: 9 FP64 additions where six butterflies take
+// 30. Lanes 4 a (a < 6) return value a's sum, a fixed tree of the lanes.
+__device__ __forceinline__ double warp_sum6(const double (&s)[6]) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+    // lanes 0-15 keep values 0, 1, 2 (and 3 in a second step), lanes 16-31 the rest: 4 + 2
+    double a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double lo = s[i], hi = i < 2 ? s[4 + i] : 0.0;  // kept by the lower / upper half
+        const double send = h16 ? lo : hi, keep = h16 ? hi : lo;
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+    double b[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const double send = h8 ? a[i] : a[2 + i], keep = h8 ? a[2 + i] : a[i];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+    const double send = h4 ? b[0] : b[1], keep = h4 ? b[1] : b[0];
+    double c = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    return c;
+}
+
 template <typename Term>
 __global__ void __launch_bounds__(kThreads) k_chunk_sums6(DevProblem P, Term term, double* __restrict__ part) {
     const int lane = threadIdx.x & 31;
@@ -545,23 +573,23 @@ __global__ void __launch_bounds__(kThreads) k_chunk_sums6(DevProblem P, Term ter
     if (c >= P.nopch) return;
     double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int q = P.opch_q[c] + lane; q < P.opch_q[c + 1]; q += 32) term(P, q, s);
-#pragma unroll
-    for (int a = 0; a < 6; ++a)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s[a] += __shfl_xor_sync(0xffffffffu, s[a], off);
-    if (lane == 0)
-#pragma unroll
-        for (int a = 0; a < 6; ++a) part[6 * c + a] = s[a];
+    __syncwarp();
+    const double v = warp_sum6(s);
+    if ((lane & 3) == 0 && lane < 24) part[6 * c + lane / 4] = v;
 }
 
 template <typename Out>
 __global__ void __launch_bounds__(kThreads) k_chunk_finish6(DevProblem P, const double* __restrict__ part, Out out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= 6LL * P.K) return;
-    const int k = (int)(i / 6), a = (int)(i % 6);
-    double v = 0.0;
-    for (int c = P.pose_opch[k]; c < P.pose_opch[k + 1]; ++c) v += part[6LL * c + a];
-    out(P, k, a, v);
+    const int lane = threadIdx.x & 31;
+    const int k = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    if (k >= P.K) return;
+    double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int c = P.pose_opch[k] + lane; c < P.pose_opch[k + 1]; c += 32)
+#pragma unroll
+        for (int a = 0; a < 6; ++a) s[a] += part[6LL * c + a];
+    __syncwarp();
+    const double v = warp_sum6(s);
+    if ((lane & 3) == 0 && lane < 24) out(P, k, lane / 4, v);
 }
 
 // part: [6 P.nopch] scratch.
@@ -572,7 +600,7 @@ void launch_pose_sums6(const DevProblem& P, double* part, Term term, Out out, cu
         k_chunk_sums6<<<grid_for(P.nopch * 32), kThreads, 0, s>>>(P, term, part);
         note_launch();
     }
-    k_chunk_finish6<<<grid_for(6LL * P.K), kThreads, 0, s>>>(P, part, out);
+    k_chunk_finish6<<<grid_for(32LL * P.K), kThreads, 0, s>>>(P, part, out);
     note_launch();
 }
 

@@ -80,10 +80,11 @@ __device__ __forceinline__ void add_rec(const double* src, double (&acc)[N]) {
 // matrix M with M X = q (0, X) q* (valid for unnormalised q),
 // M = (w^2 - |v|^2) I + 2 v v^T + 2 w [v]x, the translation, and the rotation
 // matrix of source/lie.hpp:188-204 used by the landmark Jacobian.
-// Layout per pose: M (9), t (3), R (9), pad (3).
+// Layout per pose: M (9), t (3), R in FP32 (9, in the place of 5 doubles), pad.
 constexpr int kAux = kPoseAux;
 
-__global__ void __launch_bounds__(kThreads) k_pose_aux(DevProblem P, double* aux) {
+__global__ void __launch_bounds__(kThreads) k_pose_aux(DevProblem P, double* aux, const int* __restrict__ go) {
+    if (go && !*go) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.K) return;
     const double* p = P.pose + (int64_t)k * kPoseStride;
@@ -97,14 +98,133 @@ __global__ void __launch_bounds__(kThreads) k_pose_aux(DevProblem P, double* aux
     a[10] = p[1];
     a[11] = p[2];
     const double q[4] = {w, x, y, z};
-    quat_matrix(q, a + 12);
+    double R[9];
+    quat_matrix(q, R);
+    float* rf = reinterpret_cast<float*>(a + 12);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) rf[i] = (float)R[i];
 }
 
-template <typename T>
+// The plain form's records of one observation without loss or information
+// matrix (W = I), by the zeros of the projection's Jacobian (c0, 0, c2; 0, c4,
+// c5), as in front of the camera (c2, c5 alone behind it): the same values as
+// the general code, whose products with zeros and ones are left out. FP64
+// instructions bound this kernel (a warp's holds the pipe for 64 cycles, a
+// conversion as well): some 210 instead of 330, 0.71 -> 0.53 ms at a million
+// observations.
+__device__ __forceinline__ void plain_records(const double c0, const double c2, const double c4, const double c5,
+                                              const double Xc[3], const double Rm[9], const double r[2], bool pf,
+                                              bool lf, double prec[kPoseRec], double hrec[18], double lrec[kLmRec]) {
+    const double X = Xc[0], Y = Xc[1], Z = Xc[2];
+    // rows 0 and 1 of J_p; row 0 has no entry 4, row 1 no entry 3
+    const double j0[6] = {-(c2 * Y), -(c0 * Z - c2 * X), c0 * Y, -c0, 0.0, -c2};
+    const double j1[6] = {-(c5 * Y - c4 * Z), c5 * X, -(c4 * X), 0.0, -c4, -c5};
+    double l0[3], l1[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        // (rounded as the general code's three terms with a zero among them)
+        l0[c] = -fma(c2, Rm[6 + c], __dmul_rn(c0, Rm[c]));
+        l1[c] = -fma(c5, Rm[6 + c], __dmul_rn(c4, Rm[3 + c]));
+    }
+#pragma unroll
+    for (int k = 0; k < kPoseRec; ++k) prec[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 18; ++k) hrec[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < kLmRec; ++k) lrec[k] = 0.0;
+    // u0 v0 + u1 v1 with the first or the second product fused, each as the
+    // compiler contracts the general code's expression: the results are that
+    // code's, bit for bit. (A landmark close to a camera's plane has entries
+    // that cancel to nothing in S, and another choice ends elsewhere.)
+    auto first = [](double u0, double v0, double u1, double v1) { return fma(u0, v0, __dmul_rn(u1, v1)); };
+    auto second = [](double u0, double v0, double u1, double v1) { return fma(u1, v1, __dmul_rn(u0, v0)); };
+    if (!pf) {
+        int k = 0;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+#pragma unroll
+            for (int c = a; c < 6; ++c, ++k) {
+                const bool in0 = a != 4 && c != 4, in1 = a != 3 && c != 3;
+                if (in0 && in1) prec[k] = first(j0[a], j0[c], j1[a], j1[c]);
+                else if (in0) prec[k] = j0[a] * j0[c];
+                else if (in1) prec[k] = j1[a] * j1[c];
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            if (a == 3) prec[21 + a] = -(j0[a] * r[0]);
+            else if (a == 4) prec[21 + a] = -(j1[a] * r[1]);
+            else prec[21 + a] = -second(j0[a], r[0], j1[a], r[1]);
+        }
+        if (!lf) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if (a == 3) hrec[a * 3 + c] = j0[a] * l0[c];
+                    else if (a == 4) hrec[a * 3 + c] = j1[a] * l1[c];
+                    else hrec[a * 3 + c] = second(j0[a], l0[c], j1[a], l1[c]);
+                }
+        }
+    }
+    if (!lf) {
+        lrec[0] = second(l0[0], l0[0], l1[0], l1[0]);
+        lrec[1] = second(l0[0], l0[1], l1[0], l1[1]);
+        lrec[2] = second(l0[0], l0[2], l1[0], l1[2]);
+        lrec[3] = second(l0[1], l0[1], l1[1], l1[1]);
+        lrec[4] = second(l0[1], l0[2], l1[1], l1[2]);
+        lrec[5] = second(l0[2], l0[2], l1[2], l1[2]);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) lrec[6 + a] = -second(l0[a], r[0], l1[a], r[1]);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_linearize_plain(DevProblem P, double* __restrict__ hpl,
+                                                              double* __restrict__ lm_part,
+                                                              double* __restrict__ pose_part,
+                                                              const int* __restrict__ go) {
+    if (go && !*go) return;
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // pose-major
+    if (q >= P.M) return;
+    const int64_t o = P.pose_obs[q];
+    const int pi = P.obs_pose[o], li = P.obs_lm[o];
+    const double* pp = P.pose + (int64_t)pi * kPoseStride;
+    const double* xp = P.lm + (int64_t)li * kLmStride;
+    const double2 uv = P.obs_uv[o];
+    double p[7], X[3], Xc[3], r[2], R[9];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) p[i] = __ldg(pp + i);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) X[i] = __ldg(xp + i);
+    const int front = residual(p, X, uv.x, uv.y, P.intr, Xc, r);
+    double c0 = 0.0, c2 = kBehindPenalty, c4 = 0.0, c5 = kBehindPenalty;
+    if (front) {
+        const double iz = 1.0 / Xc[2], iz2 = iz * iz;
+        c0 = P.intr.fx * iz;
+        c2 = -P.intr.fx * Xc[0] * iz2;
+        c4 = P.intr.fy * iz;
+        c5 = -P.intr.fy * Xc[1] * iz2;
+    }
+    const double qd[4] = {p[6], p[3], p[4], p[5]};
+    quat_matrix(qd, R);
+    double prec[kPoseRec], hrec[18], lrec[kLmRec];
+    plain_records(c0, c2, c4, c5, Xc, R, r, P.pose_fixed[pi] != 0, P.lm_fixed[li] != 0, prec, hrec, lrec);
+    double2* h2 = reinterpret_cast<double2*>(hpl + q * 18);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) h2[k] = make_double2(hrec[2 * k], hrec[2 * k + 1]);
+    store_rec(pose_part + q * kPoseRec, prec);
+    store_rec(lm_part + o * kLmRec, lrec);
+}
+
+// kPlain (mixed form): no loss and no information matrices; W = I, and the
+// conversions and products with it are left out (same values).
+template <typename T, bool kPlain>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(DevProblem P, T* __restrict__ hpl, T* __restrict__ lm_part,
                                                         T* __restrict__ pose_part, const double* __restrict__ aux,
-                                                        ObsJac* __restrict__ jac, float4* __restrict__ jp_pm) {
+                                                        ObsJac* __restrict__ jac, float4* __restrict__ jp_pm,
+                                                        const int* __restrict__ go) {
     constexpr int RS = RecStride<T>::value;
+    if (go && !*go) return;
     // threads in pose-major order: the large records (H_pl, pose partials)
     // are written coalesced and neighbouring threads share the pose's data.
     // In the mixed form every lane of a warp takes part in the pose sums
@@ -117,10 +237,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
     const int pi = P.obs_pose[o], li = P.obs_lm[o];
     const double* xp = P.lm + (int64_t)li * kLmStride;
     const double2 uv = P.obs_uv[o];
-    const double* om = P.obs_info ? P.obs_info + 4 * o : nullptr;
+    const double* om = !kPlain && P.obs_info ? P.obs_info + 4 * o : nullptr;
     T Jc[6], Xv, Yv, Zv, Rm[9];
     double r[2];
-    if (sizeof(T) == 8 || P.loss.kind != 0) {
+    if (sizeof(T) == 8 || (!kPlain && P.loss.kind != 0)) {
         // plain form, and the mixed form under a robust loss: residual rounded
         // exactly as the reference's. For Huber outliers rho' + 2 rho'' e2 is
         // zero in exact arithmetic and the rank-one weight term below is added
@@ -180,8 +300,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
             Jc[0] = fx * iz; Jc[1] = T(0); Jc[2] = -fx * Xv * iz2;
             Jc[3] = T(0); Jc[4] = fy * iz; Jc[5] = -fy * Yv * iz2;
         }
+        const float* rf = reinterpret_cast<const float*>(a + 12);
 #pragma unroll
-        for (int i = 0; i < 9; ++i) Rm[i] = (T)a[12 + i];
+        for (int i = 0; i < 9; ++i) Rm[i] = (T)__ldg(rf + i);
     }
 
     // Robust weight W = rho' Omega (+ 2 rho'' (Omega r)(Omega r)^T), and the
@@ -196,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
         orr1 = om[2] * r[0] + om[3] * r[1];
     }
     double drho = 1.0;
-    if (P.loss.kind) {
+    if (!kPlain && P.loss.kind) {
         const double e2 = chi2_of(r, om);
         double rho[3];
         loss_rho(P.loss, e2, rho);
@@ -228,8 +349,20 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
 #pragma unroll
         for (int c = 0; c < 3; ++c) Jl[rr * 3 + c] = -(c0 * Rm[c] + c1 * Rm[3 + c] + c2 * Rm[6 + c]);
     }
-    const T W00 = (T)Wd[0], W01 = (T)Wd[1], W10 = (T)Wd[2], W11 = (T)Wd[3];
-    const T g0 = (T)(drho * orr0), g1 = (T)(drho * orr1);
+    const T W00 = kPlain ? T(1) : (T)Wd[0], W01 = kPlain ? T(0) : (T)Wd[1], W10 = kPlain ? T(0) : (T)Wd[2],
+            W11 = kPlain ? T(1) : (T)Wd[3];
+    const double gd0 = kPlain ? r[0] : drho * orr0, gd1 = kPlain ? r[1] : drho * orr1;
+    T g0, g1;
+    df gdf0, gdf1;
+    if constexpr (sizeof(T) == 4) {  // (the double-float's first part is the rounded value)
+        gdf0 = df_from_double(gd0);
+        gdf1 = df_from_double(gd1);
+        g0 = gdf0.hi;
+        g1 = gdf1.hi;
+    } else {
+        g0 = gd0;
+        g1 = gd1;
+    }
     const bool pf = P.pose_fixed[pi] != 0, lf = P.lm_fixed[li] != 0;
 
     T prec[kPoseRec];
@@ -269,8 +402,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
         // mixed form: the Jacobian record (H_ll and b are its FP64 Gram sums)
         if (valid) {
             float4* d = reinterpret_cast<float4*>(jac + o);
-            const df g0 = df_from_double(drho * orr0), g1 = df_from_double(drho * orr1);
-            d[0] = make_float4(g0.hi, g0.lo, g1.hi, g1.lo);
+            d[0] = make_float4(gdf0.hi, gdf0.lo, gdf1.hi, gdf1.lo);
             float jp[12], jl[6];
 #pragma unroll
             for (int k = 0; k < 12; ++k) jp[k] = pf ? 0.f : (float)Jp[k];
@@ -340,8 +472,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 0) k_linearize(
 // Duplicate (pose, landmark) observations: the run's owner gets the sum of
 // the run's H_pl blocks, in order.
 template <typename T>
-__global__ void k_merge_dups(DevProblem P, T* hpl) {
+__global__ void k_merge_dups(DevProblem P, T* hpl, const int* __restrict__ go) {
     constexpr int RS = RecStride<T>::value;
+    if (go && !*go) return;
     const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (o >= P.M) return;
     if (P.dup_owner[o] != o) return;
@@ -362,7 +495,8 @@ __global__ void k_merge_dups(DevProblem P, T* hpl) {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_reduce_lm(DevProblem P, const T* __restrict__ lm_part, double* hll,
-                                                        double* b) {
+                                                        double* b, const int* __restrict__ go) {
+    if (go && !*go) return;
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= P.L) return;
     T acc[kLmRec];
@@ -444,7 +578,8 @@ __device__ __forceinline__ void store_lm_sums(const DevProblem& P, int64_t l, co
 // landmark) plus the sum carried from the previous 32 gives each landmark's
 // total in the lane holding its last observation.
 __global__ void __launch_bounds__(kThreads) k_reduce_lm_jac_thread(DevProblem P, const ObsJac* __restrict__ jac,
-                                                                   double* hll, double* b) {
+                                                                   double* hll, double* b, const int* __restrict__ go) {
+    if (go && !*go) return;
     const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (l >= P.L) return;
     df v[9];
@@ -461,7 +596,8 @@ __global__ void __launch_bounds__(kThreads) k_reduce_lm_jac_thread(DevProblem P,
 }
 
 __global__ void __launch_bounds__(kThreads) k_reduce_lm_jac(DevProblem P, const ObsJac* __restrict__ jac, double* hll,
-                                                            double* b) {
+                                                            double* b, const int* __restrict__ go) {
+    if (go && !*go) return;
     const int lane = threadIdx.x & 31;
     const int64_t ch = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (ch >= P.nlmch) return;
@@ -515,7 +651,8 @@ __global__ void __launch_bounds__(kThreads) k_reduce_lm_jac(DevProblem P, const 
 // warp order).
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_reduce_pose(DevProblem P, const T* __restrict__ pose_part, double* hpp,
-                                                          double* b) {
+                                                          double* b, const int* __restrict__ go) {
+    if (go && !*go) return;
     constexpr int NW = kThreads / 32;
     __shared__ double sh[NW][28];
     const int k = blockIdx.x;
@@ -555,7 +692,8 @@ __global__ void __launch_bounds__(kThreads) k_reduce_pose(DevProblem P, const T*
 // the chunks in turn and add in FP64; the warps' totals meet in a fixed
 // order.
 __global__ void __launch_bounds__(kThreads) k_reduce_pose_runs(DevProblem P, const float* __restrict__ pose_part,
-                                                               double* hpp, double* b) {
+                                                               double* hpp, double* b, const int* __restrict__ go) {
+    if (go && !*go) return;
     constexpr int NW = kThreads / 32;
     __shared__ double sh[NW][28];
     const int k = blockIdx.x;
@@ -1013,47 +1151,49 @@ __global__ void __launch_bounds__(kThreads) k_bs_per_pose(DevProblem P, const T*
 }
 
 // delta_l = H_ll^-1 (b_l - H_lp delta_p); delta[0..n) already holds delta_p.
-// A warp per landmark (lanes over its observations, then a butterfly: the
-// whole GPU busy at ten thousand landmarks, and a fixed order).
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_backsub(DevProblem P, const T* __restrict__ hpl,
+// Eight lanes a landmark, over its observations in turn, then a butterfly (a
+// fixed order). FP64 instructions bound it, and one costs a warp the same with
+// few lanes in use: with some 20 observations a landmark eight lanes idle
+// less than 32 and add up in three steps instead of five (165 -> 100 us at
+// 50,000 landmarks and a million observations; 58 -> 35 at 10,000 of 46).
+__global__ void __launch_bounds__(kThreads) k_backsub(DevProblem P, const double* __restrict__ hpl,
                                                       const double* __restrict__ hinv, const double* __restrict__ b,
                                                       double* delta, const LmState* st) {
-    constexpr int RS = RecStride<T>::value;
+    constexpr int kLanes = 8;
     if (!st->solve_ok) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t l = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (l >= P.L) return;
+    const int lane = threadIdx.x & (kLanes - 1);
+    const int64_t l = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kLanes;
+    const bool in = l < P.L;  // (every lane stays for the butterfly)
     double u0 = 0.0, u1 = 0.0, u2 = 0.0;
-    const int e = P.lm_ptr[l + 1];
-    for (int o = P.lm_ptr[l] + lane; o < e; o += 32) {
+    const int e = in ? P.lm_ptr[l + 1] : 0;
+    for (int o = in ? P.lm_ptr[l] + lane : 0; o < e; o += kLanes) {
         if (!P.blk_valid[o]) continue;
-        const T* h = hpl + (int64_t)P.pm[o] * RS;
+        const double* h = hpl + (int64_t)P.pm[o] * 18;
         const double* dp = delta + 6LL * P.obs_pose[o];
-        T s0 = T(0), s1 = T(0), s2 = T(0);
+        // (an observation's six terms on their own: they cancel among themselves
+        // where its block is large, and would take the sum's last bits with them)
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 #pragma unroll
         for (int a = 0; a < 6; ++a) {
-            const T d = (T)dp[a];
+            const double d = dp[a];
             s0 += h[a * 3] * d;
             s1 += h[a * 3 + 1] * d;
             s2 += h[a * 3 + 2] * d;
         }
         u0 += s0; u1 += s1; u2 += s2;
     }
+    __syncwarp();
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int off = kLanes / 2; off > 0; off >>= 1) {
         u0 += __shfl_xor_sync(0xffffffffu, u0, off);
         u1 += __shfl_xor_sync(0xffffffffu, u1, off);
         u2 += __shfl_xor_sync(0xffffffffu, u2, off);
     }
-    if (lane != 0) return;
+    if (lane >= 3 || !in) return;
+    // lane c: row c of the product with the inverse
     const double* bl = b + P.n + 3LL * l;
-    const double v0 = bl[0] - u0, v1 = bl[1] - u1, v2 = bl[2] - u2;
-    const double* I = hinv + (int64_t)l * 9;
-    double* dl = delta + P.n + 3LL * l;
-    dl[0] = I[0] * v0 + I[1] * v1 + I[2] * v2;
-    dl[1] = I[3] * v0 + I[4] * v1 + I[5] * v2;
-    dl[2] = I[6] * v0 + I[7] * v1 + I[8] * v2;
+    const double* I = hinv + (int64_t)l * 9 + 3 * lane;
+    delta[P.n + 3LL * l + lane] = I[0] * (bl[0] - u0) + I[1] * (bl[1] - u1) + I[2] * (bl[2] - u2);
 }
 
 // Backup and apply the step to free vertices.
@@ -1255,34 +1395,52 @@ long long& launch_counter() {
 constexpr int kLmThreadMin = 65536;
 
 template <typename T>
-void launch_linearize(const DevProblem& P, DevWork& W, cudaStream_t s) {
+void launch_linearize(const DevProblem& P, DevWork& W, const int* go, cudaStream_t s) {
     if (sizeof(T) == 4 && P.K > 0) {
-        k_pose_aux<<<grid_for(P.K), kThreads, 0, s>>>(P, W.pose_aux); note_launch();
+        k_pose_aux<<<grid_for(P.K), kThreads, 0, s>>>(P, W.pose_aux, go); note_launch();
     }
     if (P.M > 0) {
-        k_linearize<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl, (T*)W.lm_part, (T*)W.pose_part, W.pose_aux,
-                                                          W.jac, P.pose_win ? nullptr : W.jp_pm); note_launch();
+        const bool plain = P.loss.kind == 0 && !P.obs_info;
+        const int g = grid_for(P.M);
+        if constexpr (sizeof(T) == 8) {
+            if (plain)
+                k_linearize_plain<<<g, kThreads, 0, s>>>(P, (double*)W.hpl, (double*)W.lm_part, (double*)W.pose_part, go);
+            else
+                k_linearize<T, false><<<g, kThreads, 0, s>>>(P, (T*)W.hpl, (T*)W.lm_part, (T*)W.pose_part, nullptr,
+                                                             nullptr, nullptr, go);
+        } else {
+            float4* jp_pm = P.pose_win ? nullptr : W.jp_pm;
+            if (plain)
+                k_linearize<T, true><<<g, kThreads, 0, s>>>(P, (T*)W.hpl, (T*)W.lm_part, (T*)W.pose_part, W.pose_aux,
+                                                            W.jac, jp_pm, go);
+            else
+                k_linearize<T, false><<<g, kThreads, 0, s>>>(P, (T*)W.hpl, (T*)W.lm_part, (T*)W.pose_part, W.pose_aux,
+                                                             W.jac, jp_pm, go);
+        }
+        note_launch();
     }
-    launch_block_sums<T>(P, W, s);
+    launch_block_sums<T>(P, W, go, s);
 }
 
 template <typename T>
-void launch_block_sums(const DevProblem& P, DevWork& W, cudaStream_t s) {
-    if (P.M > 0 && P.has_dups) { k_merge_dups<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl); note_launch(); }
+void launch_block_sums(const DevProblem& P, DevWork& W, const int* go, cudaStream_t s) {
+    // (merging twice would add the duplicates twice: it has its own look at go)
+    if (P.M > 0 && P.has_dups) { k_merge_dups<T><<<grid_for(P.M), kThreads, 0, s>>>(P, (T*)W.hpl, go); note_launch(); }
     if (P.L > 0) {
         if (sizeof(T) == 4) {
             // a thread per landmark when they fill the GPU, else warps over chunks
-            if (P.L >= kLmThreadMin) k_reduce_lm_jac_thread<<<grid_for(P.L), kThreads, 0, s>>>(P, W.jac, W.hll, W.b);
-            else k_reduce_lm_jac<<<grid_for(32 * P.nlmch), kThreads, 0, s>>>(P, W.jac, W.hll, W.b);
+            if (P.L >= kLmThreadMin)
+                k_reduce_lm_jac_thread<<<grid_for(P.L), kThreads, 0, s>>>(P, W.jac, W.hll, W.b, go);
+            else k_reduce_lm_jac<<<grid_for(32 * P.nlmch), kThreads, 0, s>>>(P, W.jac, W.hll, W.b, go);
         }
-        else k_reduce_lm<T><<<grid_for(P.L), kThreads, 0, s>>>(P, (const T*)W.lm_part, W.hll, W.b);
+        else k_reduce_lm<T><<<grid_for(P.L), kThreads, 0, s>>>(P, (const T*)W.lm_part, W.hll, W.b, go);
         note_launch();
     }
     if (P.K > 0) {
         if constexpr (sizeof(T) == 4)
-            k_reduce_pose_runs<<<P.K, kThreads, 0, s>>>(P, (const float*)W.pose_part, W.hpp, W.b);
+            k_reduce_pose_runs<<<P.K, kThreads, 0, s>>>(P, (const float*)W.pose_part, W.hpp, W.b, go);
         else
-            k_reduce_pose<T><<<P.K, kThreads, 0, s>>>(P, (const T*)W.pose_part, W.hpp, W.b);
+            k_reduce_pose<T><<<P.K, kThreads, 0, s>>>(P, (const T*)W.pose_part, W.hpp, W.b, go);
         note_launch();
     }
 }
@@ -1343,10 +1501,9 @@ void launch_bs(const DevProblem& P, DevWork& W, cudaStream_t s) {
     }
 }
 
-template <typename T>
 void launch_backsub(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s) {
     if (P.L > 0) {
-        k_backsub<T><<<grid_for(32LL * P.L), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.b, W.delta, st);
+        k_backsub<<<grid_for(8LL * P.L), kThreads, 0, s>>>(P, (const double*)W.hpl, W.hll_inv, W.b, W.delta, st);
         note_launch();
     }
 }
@@ -1370,7 +1527,7 @@ void launch_cost(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, 
 }
 
 void launch_pose_aux(const DevProblem& P, DevWork& W, cudaStream_t s) {
-    if (P.K > 0) { k_pose_aux<<<grid_for(P.K), kThreads, 0, s>>>(P, W.pose_aux); note_launch(); }
+    if (P.K > 0) { k_pose_aux<<<grid_for(P.K), kThreads, 0, s>>>(P, W.pose_aux, nullptr); note_launch(); }
 }
 
 void launch_cost_fast(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, cudaStream_t s) {
@@ -1388,14 +1545,13 @@ void launch_decide(LmState* st, cudaStream_t s) { k_decide<<<1, 32, 0, s>>>(st);
 
 void launch_set_solve_ok(LmState* st, int v, cudaStream_t s) { k_set_solve_ok<<<1, 32, 0, s>>>(st, v); note_launch(); }
 
-template void launch_linearize<double>(const DevProblem&, DevWork&, cudaStream_t);
-template void launch_linearize<float>(const DevProblem&, DevWork&, cudaStream_t);
-template void launch_block_sums<double>(const DevProblem&, DevWork&, cudaStream_t);
+template void launch_linearize<double>(const DevProblem&, DevWork&, const int*, cudaStream_t);
+template void launch_linearize<float>(const DevProblem&, DevWork&, const int*, cudaStream_t);
+template void launch_block_sums<double>(const DevProblem&, DevWork&, const int*, cudaStream_t);
 template void launch_invert_w<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_invert_w<float>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_schur<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_schur<float>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
-template void launch_backsub<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_bs<double>(const DevProblem&, DevWork&, cudaStream_t);
 template void launch_bs<float>(const DevProblem&, DevWork&, cudaStream_t);
 template void launch_w<double>(const DevProblem&, DevWork&, cudaStream_t);
