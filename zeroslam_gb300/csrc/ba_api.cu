@@ -1353,8 +1353,7 @@ int pose_only_solve(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_re
         ZS_CUDA(cudaMalloc(&h->po_hist, sizeof(zs_ba_attempt) * (size_t)cap));
         h->po_hist_cap = cap;
     }
-    const int grid = pose_only_grid(h->P.M);
-    const size_t need = (size_t)grid * kPoseOnlyMaxK * 27 + (size_t)kPoseOnlyMaxK * 27 + (size_t)grid;
+    const size_t need = pose_only_scratch(h->P.M);
     if (h->po_scratch_cap < need) {
         if (h->po_scratch) ZS_CUDA(cudaFree(h->po_scratch));
         h->po_scratch = nullptr;
@@ -1362,13 +1361,10 @@ int pose_only_solve(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_re
         ZS_CUDA(cudaMalloc(&h->po_scratch, sizeof(double) * need));
         h->po_scratch_cap = need;
     }
-    double* part = h->po_scratch;
-    double* sums = part + (size_t)grid * kPoseOnlyMaxK * 27;
-    double* cpart = sums + (size_t)kPoseOnlyMaxK * 27;
     PoseOnlyCtl ctl{o.tau, o.diagonal_clamp, o.legacy_stop, o.relative_tolerance, o.chi2_floor,
                     o.max_failures, iterations, use_relative ? 1 : 0, h->po_hist_cap};
     ZS_CUDA(cudaEventRecord(h->ev0, s));
-    ZS_CUDA(launch_pose_only_lm(h->P, ctl, h->po_out, h->po_hist, part, sums, cpart, grid, s));
+    ZS_CUDA(launch_pose_only_lm(h->P, ctl, h->po_out, h->po_hist, h->po_scratch, s));
     ZS_CUDA(cudaEventRecord(h->ev1, s));
     PoseOnlyOut out{};
     ZS_CUDA(cudaMemcpyAsync(&out, h->po_out, sizeof(out), cudaMemcpyDeviceToHost, s));

@@ -149,10 +149,14 @@ __device__ inline void quat_mul_rn(const double a[4], const double b[4], double 
 __device__ inline int residual(const double* p, const double* X, double u_obs, double v_obs, const Intrinsics& in,
                                double Xc[3], double r[2]) {
     const double q[4] = {p[6], p[3], p[4], p[5]};
-    const double pq[4] = {0.0, X[0], X[1], X[2]};
     const double qc[4] = {q[0], -q[1], -q[2], -q[3]};
-    double t[4], o[4];
-    quat_mul_rn(q, pq, t);
+    // t = q (0, X): the products with the zero are left out (they change the
+    // sign of a zero at most)
+    const double t[4] = {rsub(rsub(-rmul(q[1], X[0]), rmul(q[2], X[1])), rmul(q[3], X[2])),
+                         rsub(radd(rmul(q[0], X[0]), rmul(q[2], X[2])), rmul(q[3], X[1])),
+                         radd(rsub(rmul(q[0], X[1]), rmul(q[1], X[2])), rmul(q[3], X[0])),
+                         rsub(radd(rmul(q[0], X[2]), rmul(q[1], X[1])), rmul(q[2], X[0]))};
+    double o[4];
     quat_mul_rn(t, qc, o);
     Xc[0] = radd(o[1], p[0]);
     Xc[1] = radd(o[2], p[1]);

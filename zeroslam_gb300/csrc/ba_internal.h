@@ -476,9 +476,8 @@ cudaError_t launch_preconditioner(int n, const double* S, float* F, float* X, fl
 
 // ---- pose-only problems in one launch (ba_pose_only.cu) ----
 // Every landmark fixed and at most kPoseOnlyMaxK poses: one cooperative
-// launch of `grid` CTAs (pose_only_grid(M)) runs the whole LM loop (FP64) on
-// the poses in P.pose. Device memory: out, hist (hist_cap attempt records),
-// part [grid * K * 27], sums [K * 27], cpart [grid].
+// launch runs the whole LM loop (FP64) on the poses in P.pose. Device memory:
+// out, hist (hist_cap attempt records), scratch (pose_only_scratch(M) doubles).
 constexpr int kPoseOnlyMaxK = 64;
 // At most this many free poses: each free pose's sums take one pass of the
 // grid (the FP64 pipe bounds it), so problems with more free poses are
@@ -492,14 +491,14 @@ struct PoseOnlyOut {
     int iterations, attempts, accepted, cholesky_failures, history;
     double chi2_initial, chi2_final, lambda_final;
 };
-int pose_only_grid(int64_t M);
+size_t pose_only_scratch(int64_t M);
 // A batch whose landmarks are all fixed: one CTA per window (at most
 // kPoseOnlyMaxK poses each), reports into wctl / wst as the general batched
 // path's per-window control and state.
 cudaError_t launch_pose_only_windows(const DevProblem& P, const PoseOnlyCtl& ctl, WinCtl* wctl, LmState* wst,
                                     cudaStream_t s);
 cudaError_t launch_pose_only_lm(const DevProblem& P, const PoseOnlyCtl& ctl, PoseOnlyOut* out, zs_ba_attempt* hist,
-                                double* part, double* sums, double* cpart, int grid, cudaStream_t s);
+                                double* scratch, cudaStream_t s);
 
 // ---- FP32 products on the tensor cores (ba_tc_gemm.cu) ----
 // C (M x N, row stride ldc) = alpha A B^T + beta C, A (M x K) and B (N x K)
