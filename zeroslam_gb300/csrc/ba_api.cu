@@ -375,6 +375,7 @@ struct zs_ba_handle {
     // batched windows
     bool batch = false;
     BatchDev B;
+    FxBatch bfx;
     std::vector<int32_t> wpose0, wlm0;  // first pose / landmark of each window, plus the end
     cudaGraph_t bgraph = nullptr;
     cudaGraphExec_t bexec = nullptr;
@@ -1937,7 +1938,7 @@ int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* Lou
 namespace {
 
 // Version of the window-solve kernel the tuning results belong to.
-constexpr const char* kTuneKernel = "bsolve-tiles32-v2";
+constexpr const char* kTuneKernel = "bsolve-tiles32-v3";
 
 // Autotuned reduced-solve block sizes per (device name, precision, bucket),
 // shared by all handles of the process and optionally kept in a file:
@@ -2159,13 +2160,15 @@ int solve_batch_impl(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_r
     r.kernel_launches = r.graph_launches ? h->bpro_launches + (long long)rounds * h->bbody_launches
                                          : launch_counter() - launches0;
     int64_t accepted = 0;
+    r.status = ZS_OK;
     for (int w = 0; w < P.nwin; ++w) {
         accepted += ctl[w].accepted;
+        if (st[w].timeout) r.status = ZS_ERR_TIMEOUT;
         r.attempts += ctl[w].attempts;
         if (!wr) continue;
         zs_ba_report& o = wr[w];
         std::memset(&o, 0, sizeof(o));
-        o.status = ZS_OK;
+        o.status = st[w].timeout ? ZS_ERR_TIMEOUT : ZS_OK;
         o.iterations = ctl[w].iterations;
         o.accepted = ctl[w].accepted;
         o.attempts = ctl[w].attempts;
@@ -2177,8 +2180,11 @@ int solve_batch_impl(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_r
         o.ms_total = ms;
     }
     r.accepted = accepted;
-    r.status = ZS_OK;
     if (rep) *rep = r;
+    if (r.status == ZS_ERR_TIMEOUT) {
+        std::snprintf(g_last_error, sizeof(g_last_error), "a dependency wait of a window's factor ran out");
+        return ZS_ERR_TIMEOUT;
+    }
     return (int)std::min<int64_t>(accepted, 0x7fffffff);
 }
 
@@ -2275,6 +2281,27 @@ int zs_ba_set_batch(zs_ba_handle* h, int num_windows, const zs_ba_problem* windo
             ZS_CUDA(cudaEventCreateWithFlags(&B.ev_join[b], cudaEventDisableTiming));
         }
         B.lists = upload(lists, own, h->stream);
+        B.fx = nullptr;
+        if (h->tsize == 8) {
+            std::vector<int> wn(num_windows);
+            std::vector<int64_t> ws(num_windows);
+            int64_t at = 0;
+            for (int w = 0; w < num_windows; ++w) {
+                wn[w] = 6 * (wp[w + 1] - wp[w]);
+                ws[w] = at;  // (as P.win_s_off)
+                at += (int64_t)wn[w] * wn[w];
+            }
+            std::vector<FxWindow> win;
+            std::vector<uint32_t> tasks;
+            const size_t bytes = fx_batch_plan(wn, ws, win, tasks);
+            h->bfx = FxBatch{};
+            h->bfx.win = upload(win, own, h->stream);
+            h->bfx.tasks = upload(tasks, own, h->stream);
+            h->bfx.ntasks = (int)tasks.size();
+            h->bfx.work = dalloc<char>(std::max<size_t>(bytes, 1), own);
+            h->bfx.next = dalloc<int>(1, own);
+            B.fx = &h->bfx;
+        }
         B.st = dalloc<LmState>(num_windows, own);
         B.ctl = dalloc<WinCtl>(num_windows, own);
         B.counters = dalloc<int>(kBatchBuckets, own);

@@ -8,12 +8,15 @@
 //     same acceptance, damping, rollback and stop rules as zs_ba_solve;
 //   * the damped H_ll inverses and S block initialisation at each window's
 //     own lambda (the pair products go into the window's S block);
-//   * the reduced solve: a persistent kernel per size bucket whose CTAs
-//     take windows from a device work queue (largest first), factor the
-//     window's S in shared memory (packed lower triangle, right-looking
-//     Cholesky with the reference's pivot and solve thresholds,
-//     source/matrix_decomposition_cholesky.hpp:26-95), solve with one warp,
-//     and in the mixed form refine against the FP64 S;
+//   * the reduced solve. In the plain form one launch factors all windows'
+//     systems in fixed point, a task per 32 x 32 tile (k_chol_fx_windows,
+//     ba_chol_fx.cu); then, in both forms, a persistent kernel per size
+//     bucket whose CTAs take windows from a device work queue (largest
+//     first): the mixed form's factors the window's S in shared memory
+//     (packed lower triangle, right-looking Cholesky with the reference's
+//     pivot and solve thresholds, source/matrix_decomposition_cholesky.hpp:26-95),
+//     solves with it and refines against the FP64 S, the plain form's makes
+//     the solve test and solves;
 //   * per-window cost and model-decrease sums in a fixed order.
 // A round's kernels are captured once into a CUDA graph body that a
 // conditional WHILE node repeats until no window is active, so a batched
@@ -284,6 +287,7 @@ __global__ void __launch_bounds__(kThreads) k_binit(DevProblem P, const double* 
     s.good = 0;
     s.rho = 0.0;
     s.refine_sweeps = 0;
+    s.timeout = 0;
     WinCtl& c = ctl[w];
     const bool has_obs = P.win_ochunk[w + 1] > P.win_ochunk[w];
     c.active = (prm.iterations > 0 && prm.max_failures > 0 && has_obs && (p1 > p0 || l1 > l0)) ? 1 : 0;
@@ -324,6 +328,11 @@ __global__ void __launch_bounds__(kThreads) k_bdecide(int nwin, LmState* st, Win
             s.good = 0;
             c.failures++;
             end_inner = !isfinite(s.lambda) || c.failures >= prm.max_failures;
+            if (s.timeout) {  // a bounded wait of the factor ran out: the window stops where it is
+                c.active = 0;
+                c.iterations = c.it + 1;
+                end_inner = false;
+            }
         } else {
             c.refine_sweeps += s.refine_sweeps;
             const double rho = (s.chi2 - s.chi2_new) / s.scale;
@@ -402,11 +411,15 @@ constexpr size_t bsolve_smem() {
 }
 
 // Persistent reduced solve of one size bucket: CTAs take windows from the
-// bucket's queue (list, largest first). Per window: S_w (FP64, global) ->
-// tiles in shared memory (TF), blocked Cholesky with pivot test
+// bucket's queue (list, largest first). Per window, the plain form: S_w holds
+// its factor L (k_chol_fx_windows; 64 windows of up to 30 poses took 1.0 ms a
+// round with an FP64 factor by this kernel, bound by one warp's FP64 chain,
+// and now take 0.15 ms and these solves), the reference's solve test and the
+// solves. The mixed form: S_w (FP64, global) -> tiles in shared memory (TF),
+// blocked Cholesky with pivot test
 // d > 1e-14 max|S_ii| and solve test |L_ii| > 1e-7 max|L_ii|
 // (source/matrix_decomposition_cholesky.hpp:40,53,74,80,89), blocked
-// triangular solves; with refine_iters > 0, FP64 refinement
+// triangular solves; FP64 refinement
 // x += (L L^T)^-1 (b - S x) until ||b - S x|| <= tol ||b||.
 template <typename TF, int NB>
 __global__ void k_bsolve(BatchView V, const int32_t* __restrict__ list, int count, int* counter, int refine_iters,
@@ -432,6 +445,10 @@ __global__ void k_bsolve(BatchView V, const int32_t* __restrict__ list, int coun
         if (idx >= count) return;
         const int w = list[idx];
         if (!V.ctl[w].active) continue;
+        if (sizeof(TF) == 8 && !V.st[w].solve_ok) {  // the factor failed
+            if (tid == 0) V.st[w].refine_sweeps = 0;
+            continue;
+        }
         long long t0 = V.prof ? clock64() : 0;
         const int p0 = V.win_pose0[w];
         const int n = 6 * (V.win_pose0[w + 1] - p0);
@@ -497,7 +514,18 @@ __global__ void k_bsolve(BatchView V, const int32_t* __restrict__ list, int coun
             }
         };
         mark(0);
-        int ok = cta_cholesky<TF>(A, nbw, n, eps, dinv, &s_flag);
+        int ok = 1;
+        if constexpr (kScale) {
+            ok = cta_cholesky<TF>(A, nbw, n, eps, dinv, &s_flag);
+        } else {  // the tiles are L already: what the solves need of the diagonal tiles
+            for (int kb = warp; kb < nbw; kb += nwarps) {
+                TF* D = tile_at(A, kb, kb);
+                dinv[32 * kb + lane] = TF(1) / D[lane * kLd + lane];
+                __syncwarp();
+                warp_tile_inverse(D, dinv + 32 * kb);
+            }
+            __syncthreads();
+        }
         int sweeps = 0;
         if (ok) {
             // solve test on the unscaled diagonal L_ii = Ltilde_ii / sc_i
@@ -659,6 +687,10 @@ cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, con
     }
     launch_schur_pairs<T>(P, W, B.ctl, s);
     launch_bs<T>(P, W, s);
+    if (B.fx) {
+        const cudaError_t e = launch_chol_fx_windows(*B.fx, P.nwin, W.S, B.st, B.ctl, s);
+        if (e != cudaSuccess) return e;
+    }
     BatchView V{W.S, W.bs, W.delta, B.st, B.ctl, P.win_pose0, P.win_s_off, B.prof};
     const int refine = sizeof(T) == 4 ? prm.refine_iters : 0;
     cudaError_t e = cudaEventRecord(B.ev_fork, s);
@@ -711,6 +743,7 @@ __global__ void k_tune_fill(int n, int nwin, double* S, double* bs, LmState* st,
         ctl[idx] = WinCtl{};
         ctl[idx].active = 1;
         st[idx] = LmState{};
+        st[idx].solve_ok = 1;  // (the plain form solves with S as if it were the factor)
         pose0[idx] = (int32_t)(idx * (n / 6));
         soff[idx] = idx * nn;
         list[idx] = (int32_t)idx;

@@ -42,6 +42,7 @@
 // wait returns), st->timeout set and st->solve_ok cleared.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "ba_fixed.cuh"
@@ -696,11 +697,56 @@ __global__ void __launch_bounds__(kFxThreads, 2) k_chol_fx(Fx d) {
     }
 }
 
-// eps_factor = 1e-14 max |S_ii|, the rows' scales, cleared flags. A diagonal
-// entry at most eps fails at once: its pivot cannot exceed it.
-__global__ void __launch_bounds__(1024) k_fx_prepare(int n, int rows, const double* __restrict__ S, int* e, int* flags,
-                                                     int nflags, LmState* st) {
+// A batch of windows: the same tiles, tasks (window, i, j) column by column
+// over all windows, largest window first, taken from a queue. Whoever took a
+// task's dependencies runs or has finished, so the lowest unfinished task can
+// proceed whatever the grid. A window that fails or is not active is passed
+// over by its abort flag.
+__global__ void __launch_bounds__(kFxThreads, 2) k_chol_fx_windows(const FxWindow* __restrict__ win,
+                                                                   const uint32_t* __restrict__ tasks, int ntasks,
+                                                                   int* next, char* work, double* S, LmState* st,
+                                                                   int stall) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Smem<32>& sm = *reinterpret_cast<Smem<32>*>(smem_raw);
+    __shared__ int s_task;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_task = atomicAdd(next, 1);
+        __syncthreads();
+        const int t = s_task;
+        if (t >= ntasks) return;
+        const uint32_t task = tasks[t];
+        const int w = (int)(task >> 8), i = (int)(task >> 4 & 15), j = (int)(task & 15);
+        const FxWindow v = win[w];
+        const FxLayout l = fx_layout(v.n);
+        char* base = work + v.work;
+        Fx d;
+        d.n = v.n;
+        d.N = l.N;
+        d.S = S + v.s;
+        d.F = S + v.s;  // (an entry is read by the one CTA that writes it, before it does)
+        d.Q = reinterpret_cast<int2*>(base);
+        d.G = reinterpret_cast<int2*>(base + l.g);
+        d.e = reinterpret_cast<const int*>(base + l.e);
+        d.f = reinterpret_cast<int4*>(base + l.f);
+        d.flag = reinterpret_cast<int*>(base + l.flag);
+        d.abort = d.flag + l.tiles;
+        d.st = st + w;
+        d.stall = stall;
+        if (__syncthreads_or(threadIdx.x == 0 && ld_acquire(d.abort) != 0)) continue;
+        if (i == j) task_diag<32>(d, j, t, sm);
+        else if (i == j + 1) task_tile<32, true>(d, i, j, t, sm);
+        else task_tile<32, false>(d, i, j, t, sm);
+    }
+}
+
+// eps_factor = 1e-14 max |S_ii|, the rows' scales, cleared flags (the last one
+// is the abort flag). A diagonal entry at most eps fails at once: its pivot
+// cannot exceed it. Returns whether one did (in thread 0).
+__device__ int fx_prepare(int n, int rows, const double* S, int* e, int* flags, int nflags, LmState* st) {
     __shared__ double sh[32];
+    if (threadIdx.x < 32) sh[threadIdx.x] = 0.0;
+    __syncthreads();
     double m = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, fabs(S[(int64_t)i * n + i]));
 #pragma unroll
@@ -724,10 +770,32 @@ __global__ void __launch_bounds__(1024) k_fx_prepare(int n, int rows, const doub
     }
     for (int i = threadIdx.x; i < nflags; i += blockDim.x) flags[i] = 0;
     if (__syncthreads_or(bad)) bad = 1;
-    if (threadIdx.x == 0) {
-        st->eps_factor = eps;
-        if (bad) st->solve_ok = 0;
+    if (threadIdx.x == 0) st->eps_factor = eps;
+    return bad;
+}
+
+__global__ void __launch_bounds__(1024) k_fx_prepare(int n, int rows, const double* __restrict__ S, int* e, int* flags,
+                                                     int nflags, LmState* st) {
+    if (fx_prepare(n, rows, S, e, flags, nflags, st) && threadIdx.x == 0) st->solve_ok = 0;
+}
+
+// A CTA per window; st->solve_ok of active windows is set here.
+__global__ void __launch_bounds__(128) k_fx_prepare_windows(const FxWindow* __restrict__ win, int* next, char* work,
+                                                            const double* __restrict__ S, LmState* st,
+                                                            const WinCtl* __restrict__ ctl) {
+    const int w = blockIdx.x;
+    if (w == 0 && threadIdx.x == 0) *next = 0;
+    const FxWindow v = win[w];
+    const FxLayout l = fx_layout(v.n);
+    char* base = work + v.work;
+    int* flag = reinterpret_cast<int*>(base + l.flag);
+    int skip = 1;
+    if (ctl[w].active) {
+        skip = fx_prepare(v.n, l.N * l.T, S + v.s, reinterpret_cast<int*>(base + l.e), flag, l.tiles + 1, st + w);
+        if (threadIdx.x == 0) st[w].solve_ok = !skip;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) flag[l.tiles] = skip;
 }
 
 int stall_task_from_env() {
@@ -735,19 +803,22 @@ int stall_task_from_env() {
     return v && *v ? std::atoi(v) : -1;
 }
 
+// CTAs of the kernel that are resident together (0: an error is pending).
+int resident_ctas(const void* kernel, size_t smem) {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFxThreads, smem) != cudaSuccess)
+        return 0;
+    return sms * per_sm;
+}
+
 template <int T>
 cudaError_t launch_fx(Fx& d, int tasks, cudaStream_t s) {
     static std::atomic<int> resident[kMaxDevices];
     const size_t smem = sizeof(Smem<T>);
-    const int co = per_device(resident, [&] {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaFuncSetAttribute(k_chol_fx<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chol_fx<T>, kFxThreads, smem) != cudaSuccess)
-            return 0;
-        return sms * per_sm;
-    });
+    const int co = per_device(resident, [&] { return resident_ctas((const void*)k_chol_fx<T>, smem); });
     if (co < 1) {
         const cudaError_t e = cudaGetLastError();
         return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
@@ -782,6 +853,51 @@ cudaError_t launch_chol_fx(int n, const double* S, double* F, void* work, LmStat
     d.stall = stall;
     k_fx_prepare<<<1, 1024, 0, s>>>(n, l.N * l.T, S, e, d.flag, l.tiles + 1, st); note_launch();
     return l.T == 32 ? launch_fx<32>(d, l.tiles, s) : launch_fx<64>(d, l.tiles, s);
+}
+
+size_t fx_batch_plan(const std::vector<int>& n, const std::vector<int64_t>& s, std::vector<FxWindow>& win,
+                     std::vector<uint32_t>& tasks) {
+    win.assign(n.size(), FxWindow{});
+    tasks.clear();
+    size_t bytes = 0;
+    std::vector<int> order(n.size());
+    for (size_t w = 0; w < n.size(); ++w) {
+        win[w] = {n[w], s[w], (int64_t)bytes};
+        bytes += (chol_fx_bytes(n[w]) + 255) / 256 * 256;
+        order[w] = (int)w;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
+    const int most = order.empty() ? 0 : fx_layout(n[order[0]]).N;
+    for (int j = 0; j < most; ++j)
+        for (int d = 0; j + d < most; ++d)  // (every window's diagonal tile, then the tiles below it)
+            for (int w : order) {
+                const int i = j + d;
+                if (i >= fx_layout(n[w]).N) break;
+                if (d == 0 && j > 0) break;  // with tile (j, j - 1)
+                tasks.push_back((uint32_t)w << 8 | (uint32_t)i << 4 | (uint32_t)j);
+            }
+    return bytes;
+}
+
+cudaError_t launch_chol_fx_windows(const FxBatch& b, int nwin, double* S, LmState* st, const WinCtl* ctl,
+                                   cudaStream_t s) {
+    if (nwin < 1) return cudaSuccess;
+    static const int stall = stall_task_from_env();
+    static std::atomic<int> resident[kMaxDevices];
+    const size_t smem = sizeof(Smem<32>);
+    const int co = per_device(resident, [&] { return resident_ctas((const void*)k_chol_fx_windows, smem); });
+    if (co < 1) {
+        const cudaError_t e = cudaGetLastError();
+        return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+    }
+    k_fx_prepare_windows<<<nwin, 128, 0, s>>>(b.win, b.next, b.work, S, st, ctl);
+    note_launch();
+    if (b.ntasks > 0) {
+        k_chol_fx_windows<<<std::min(b.ntasks, co), kFxThreads, smem, s>>>(b.win, b.tasks, b.ntasks, b.next, b.work, S,
+                                                                          st, stall);
+        note_launch();
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace zs

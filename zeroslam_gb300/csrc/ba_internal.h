@@ -280,6 +280,7 @@ struct BatchView {
 // load, factor, first solve, refinement, refinement sweeps
 constexpr int kBatchProfSlots = 5;
 
+struct FxBatch;
 struct BatchDev {
     LmState* st = nullptr;       // [nwin]
     WinCtl* ctl = nullptr;       // [nwin]
@@ -291,6 +292,7 @@ struct BatchDev {
     int bucket_off[kBatchBuckets + 1] = {0};
     int threads[kBatchBuckets] = {0};
     int blocks[kBatchBuckets] = {0};
+    FxBatch* fx = nullptr;       // plain form: the windows' factors
     // the buckets' reduced solves run concurrently: forked from the main
     // stream by ev_fork, joined back by ev_join
     cudaStream_t streams[kBatchBuckets] = {nullptr};
@@ -418,6 +420,24 @@ constexpr size_t chol_fx_bytes(int n) { return fx_layout(n > 0 ? n : 1).bytes; }
 // S (n x n row-major, its lower triangle read) -> F = L (lower triangle
 // written); st->solve_ok = 0 on a failed pivot.
 cudaError_t launch_chol_fx(int n, const double* S, double* F, void* work, LmState* st, cudaStream_t s);
+// The factors of a batch's active windows in place (each window's S at S + s,
+// n <= 6 kBatchMaxK), st[w].solve_ok set.
+struct FxWindow {
+    int n;
+    int64_t s, work;  // offsets: doubles into S, bytes into the workspace
+};
+struct FxBatch {
+    FxWindow* win = nullptr;    // [nwin]
+    uint32_t* tasks = nullptr;  // [ntasks] window << 8 | i << 4 | j
+    int ntasks = 0;
+    char* work = nullptr;
+    int* next = nullptr;  // [1] the tasks' queue
+};
+// The windows' places and tasks; returns the workspace's bytes.
+size_t fx_batch_plan(const std::vector<int>& n, const std::vector<int64_t>& s, std::vector<FxWindow>& win,
+                     std::vector<uint32_t>& tasks);
+cudaError_t launch_chol_fx_windows(const FxBatch& b, int nwin, double* S, LmState* st, const WinCtl* ctl,
+                                   cudaStream_t s);
 
 // ---- mixed form: the preconditioner (ba_chol_dag.cu) ----
 // F (n x n FP32, the matrix) -> L in F's lower triangle (zeros above the

@@ -33,19 +33,35 @@ __device__ __forceinline__ TF* tile_at(TF* A, int ib, int jb) {
 // is the reference's test on the unscaled pivot
 // (source/matrix_decomposition_cholesky.hpp:40,53).
 // Returns 1 on success (uniform over the CTA).
-// Pivot d -> (L_cc, 1 / L_cc). The mixed form (float) uses the reciprocal
-// square root (its refinement corrects the factor's last bits); the plain
-// form keeps the reference's sqrt and division.
+// Pivot d -> (L_cc, 1 / L_cc) by the reciprocal square root (the mixed form's
+// refinement corrects the factor's last bits).
 __device__ __forceinline__ void pivot_root(float d, float& l, float& inv) {
     inv = rsqrtf(d);
     l = d * inv;
 }
-__device__ __forceinline__ void pivot_root(double d, double& l, double& inv) {
-    l = sqrt(d);
-    inv = 1.0 / l;
+
+// One warp: the diagonal tile D = L_kk's inverse, transposed, into its upper
+// triangle: column `lane` of L_kk^-1, right-looking. dinv: the tile's 1 / L_ii.
+template <typename TF>
+__device__ __forceinline__ void warp_tile_inverse(TF* D, const TF* dinv) {
+    const int lane = threadIdx.x & 31;
+    TF acc[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = TF(0);
+#pragma unroll
+    for (int m = 0; m < 32; ++m) {
+        const TF dm = dinv[m];
+        const TF ym = (m < lane) ? TF(0) : ((m == lane) ? dm : -acc[m] * dm);
+        acc[m] = ym;  // acc[m] now holds y_m
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (i > m) acc[i] += D[i * kLd + m] * ym;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        if (i > lane) D[lane * kLd + i] = acc[i];
 }
-__device__ __forceinline__ float scale_by(float x, float l, float inv) { return x * inv; }
-__device__ __forceinline__ double scale_by(double x, double l, double inv) { return x / l; }
 
 template <typename TF>
 __device__ int cta_cholesky(TF* A, int nbw, int n, const TF* eps, TF* dinv, int* s_flag) {
@@ -69,7 +85,7 @@ __device__ int cta_cholesky(TF* A, int nbw, int n, const TF* eps, TF* dinv, int*
                     row[c] = lcc;
                     own_inv = inv;
                 }
-                if (lane > c) row[c] = scale_by(row[c], lcc, inv);
+                if (lane > c) row[c] = row[c] * inv;
                 const TF lic = row[c];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
@@ -84,23 +100,7 @@ __device__ int cta_cholesky(TF* A, int nbw, int n, const TF* eps, TF* dinv, int*
                 if (j <= lane) D[lane * kLd + j] = row[j];
             dinv[32 * kb + lane] = own_inv;  // 1 / L_ii of this tile
             __syncwarp();
-            // column `lane` of L_kk^-1, right-looking
-            TF acc[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = TF(0);
-#pragma unroll
-            for (int m = 0; m < 32; ++m) {
-                const TF dm = dinv[32 * kb + m];
-                const TF ym = (m < lane) ? TF(0) : ((m == lane) ? dm : -acc[m] * dm);
-                acc[m] = ym;  // acc[m] now holds y_m
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (i > m) acc[i] += D[i * kLd + m] * ym;
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                if (i > lane) D[lane * kLd + i] = acc[i];
+            warp_tile_inverse(D, dinv + 32 * kb);
             if (lane == 0) *s_flag = fail;
         }
         __syncthreads();
