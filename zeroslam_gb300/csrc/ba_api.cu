@@ -348,6 +348,40 @@ T* upload(const HostArray<T>& v, DevPool& pool, cudaStream_t s) {
     return d;
 }
 
+// A copy of its own costs about 6 us of the calling thread, and 4 us more from
+// or to pageable memory, whatever its size; the CPU writes 64 KB to pinned
+// memory in 1 us, but 1 MB in 32 us, where a copy takes 12. So arrays up to
+// 64 KB travel together through one pinned buffer of the handle, larger ones
+// by themselves (a tracked frame, 24 arrays of 1,312 observations: 575 -> 501 us
+// for the whole map_optimise call; matching 2,000 descriptors: 80 -> 76).
+constexpr size_t kSmallCopy = 64 << 10;
+constexpr size_t kStage = 512 << 10;
+
+// The small host arrays of one upload, packed into `host` (pinned, kStage
+// bytes, free until the stream has been synchronised) and one device buffer.
+struct PackedUpload {
+    DevPool& pool;
+    cudaStream_t s;
+    char* host;
+    char* dev;
+    size_t used = 0;
+    PackedUpload(DevPool& p, cudaStream_t st, char* h) : pool(p), s(st), host(h), dev(dalloc<char>(kStage, p)) {}
+    template <typename V>
+    auto put(const V& v) {
+        using T = std::remove_cv_t<std::remove_pointer_t<decltype(v.data())>>;
+        const size_t bytes = v.size() * sizeof(T);
+        if (bytes > kSmallCopy || used + bytes > kStage) return upload(v, pool, s);
+        pool.get(0);  // (the array's place in the pool's order)
+        if (bytes) std::memcpy(host + used, v.data(), bytes);
+        T* d = reinterpret_cast<T*>(dev + used);
+        used = std::min(kStage, (used + bytes + 255) & ~size_t(255));
+        return d;
+    }
+    void flush() {
+        if (used) ZS_CUDA(cudaMemcpyAsync(dev, host, used, cudaMemcpyHostToDevice, s));
+    }
+};
+
 }  // namespace
 
 struct zs_ba_handle {
@@ -369,6 +403,11 @@ struct zs_ba_handle {
     std::vector<int64_t> perm;   // landmark-major position -> caller's observation index
     int tsize = 8;
     HostScratch hscratch;        // build_problem's host arrays (pinned, reused)
+    HostScratch hstage;          // small copies (pinned, kStage bytes)
+    char* stage() {
+        hstage.next = 0;
+        return static_cast<char*>(hstage.get(kStage));
+    }
     std::vector<zs_ba_attempt> history;  // the last single-problem solve's attempts
     void* aux_buf = nullptr;     // device arrays of map culling and matching (handle lifetime, grown on demand)
     size_t aux_cap = 0;
@@ -392,7 +431,7 @@ struct zs_ba_handle {
     PoseOnlyOut* po_out = nullptr;
     zs_ba_attempt* po_hist = nullptr;
     int po_hist_cap = 0;
-    double* po_scratch = nullptr;  // partial sums: [grid * 64 * 27] + [64 * 27] + [grid]
+    double* po_scratch = nullptr;  // partial sums (pose_only_scratch)
     size_t po_scratch_cap = 0;
 
     void release_graph() {
@@ -581,9 +620,9 @@ void zs_ba_destroy(zs_ba_handle* h) {
     h->timer.destroy();
     h->release_problem();
     h->hscratch.release();
+    h->hstage.release();
     if (h->aux_buf) cudaFree(h->aux_buf);
     if (h->po_out) cudaFree(h->po_out);
-    if (h->po_hist) cudaFree(h->po_hist);
     if (h->po_scratch) cudaFree(h->po_scratch);
     if (h->st) cudaFree(h->st);
     if (h->st_host) cudaFreeHost(h->st_host);
@@ -900,36 +939,37 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
     for (int k = 0; k < K; ++k) h->free_poses += pf[k] == 0;
 
     auto& own = h->owned;
-    P.pose = upload(pose8, own, s);
+    PackedUpload up(own, s, h->stage());
+    P.pose = up.put(pose8);
     P.pose_bk = dalloc<double>(pose8.size(), own);
-    P.lm = upload(lm4, own, s);
+    P.lm = up.put(lm4);
     P.lm_bk = dalloc<double>(lm4.size(), own);
-    P.pose_init = upload(pose8, own, s);
-    P.lm_init = upload(lm4, own, s);
-    P.pose_fixed = upload(pf, own, s);
-    P.lm_fixed = upload(lf, own, s);
-    P.obs_pose = upload(obs_pose, own, s);
-    P.obs_lm = upload(obs_lm, own, s);
-    P.obs_uv = upload(uv, own, s);
-    P.obs_info = p->obs_info ? upload(info, own, s) : nullptr;
-    P.lm_ptr = upload(lm_ptr, own, s);
-    P.pose_ptr = upload(pose_ptr, own, s);
-    P.pose_obs = upload(pose_obs, own, s);
-    P.blk_valid = upload(blk_valid, own, s);
+    P.pose_init = up.put(pose8);
+    P.lm_init = up.put(lm4);
+    P.pose_fixed = up.put(pf);
+    P.lm_fixed = up.put(lf);
+    P.obs_pose = up.put(obs_pose);
+    P.obs_lm = up.put(obs_lm);
+    P.obs_uv = up.put(uv);
+    P.obs_info = p->obs_info ? up.put(info) : nullptr;
+    P.lm_ptr = up.put(lm_ptr);
+    P.pose_ptr = up.put(pose_ptr);
+    P.pose_obs = up.put(pose_obs);
+    P.blk_valid = up.put(blk_valid);
     P.has_dups = has_dups;
-    P.dup_owner = has_dups ? upload(dup_owner, own, s) : nullptr;
-    P.pair_i = upload(pair_i, own, s);
-    P.pair_j = upload(pair_j, own, s);
-    P.seg_ptr = upload(seg_ptr, own, s);
-    P.seg_pair = upload(seg_pair, own, s);
-    P.pair_seg_ptr = upload(pair_seg_ptr, own, s);
-    P.pm = upload(pm, own, s);
+    P.dup_owner = has_dups ? up.put(dup_owner) : nullptr;
+    P.pair_i = up.put(pair_i);
+    P.pair_j = up.put(pair_j);
+    P.seg_ptr = up.put(seg_ptr);
+    P.seg_pair = up.put(seg_pair);
+    P.pair_seg_ptr = up.put(pair_seg_ptr);
+    P.pm = up.put(pm);
     P.nopch = (int64_t)opch_q.size() - 1;
-    P.opch_q = upload(opch_q, own, s);
-    P.pose_opch = upload(pose_opch, own, s);
+    P.opch_q = up.put(opch_q);
+    P.pose_opch = up.put(pose_opch);
     P.nlmch = (int64_t)lmch_l.size() - 1;
-    P.lmch_l = upload(lmch_l, own, s);
-    P.triples = upload(triples, own, s);
+    P.lmch_l = up.put(lmch_l);
+    P.triples = up.put(triples);
     stamp("uploads");
     P.nwin = nwin;
     std::vector<int64_t> win_s_off(nwin, 0);
@@ -952,16 +992,17 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
             win_ochunk.push_back((int32_t)ochunk_win.size());
         }
         P.nochunks = (int64_t)ochunk_win.size();
-        P.pose_win = upload(pose_win, own, s);
-        P.lm_win = upload(lm_win, own, s);
-        P.win_pose0 = upload(wp, own, s);
-        P.win_lm0 = upload(wl, own, s);
-        P.win_s_off = upload(win_s_off, own, s);
-        P.ochunk_ptr = upload(ochunk_ptr, own, s);
-        P.ochunk_win = upload(ochunk_win, own, s);
-        P.win_ochunk = upload(win_ochunk, own, s);
+        P.pose_win = up.put(pose_win);
+        P.lm_win = up.put(lm_win);
+        P.win_pose0 = up.put(wp);
+        P.win_lm0 = up.put(wl);
+        P.win_s_off = up.put(win_s_off);
+        P.ochunk_ptr = up.put(ochunk_ptr);
+        P.ochunk_win = up.put(ochunk_win);
+        P.win_ochunk = up.put(win_ochunk);
     }
 
+    up.flush();
     const size_t ts = (size_t)h->tsize;
     const int n = P.n;
     DevWork& W = h->W;
@@ -1072,6 +1113,21 @@ int zs_ba_get_state(zs_ba_handle* h, double* poses, double* landmarks) {
     const DevProblem& P = h->P;
     try {
         ZS_CUDA(cudaSetDevice(h->device));
+        const size_t pb = poses ? sizeof(double) * kPoseStride * (size_t)P.K : 0;
+        const size_t lb = landmarks ? sizeof(double) * kLmStride * (size_t)P.L : 0;
+        if (pb + lb <= 2 * kSmallCopy) {
+            char* st = h->stage();
+            if (pb) ZS_CUDA(cudaMemcpyAsync(st, P.pose, pb, cudaMemcpyDeviceToHost, h->stream));
+            if (lb) ZS_CUDA(cudaMemcpyAsync(st + pb, P.lm, lb, cudaMemcpyDeviceToHost, h->stream));
+            ZS_CUDA(cudaStreamSynchronize(h->stream));
+            const double* sp = reinterpret_cast<const double*>(st);
+            const double* sl = reinterpret_cast<const double*>(st + pb);
+            for (int k = 0; pb && k < P.K; ++k)
+                std::memcpy(poses + 7 * (int64_t)k, sp + kPoseStride * (int64_t)k, 7 * sizeof(double));
+            for (int l = 0; lb && l < P.L; ++l)
+                std::memcpy(landmarks + 3 * (int64_t)l, sl + kLmStride * (int64_t)l, 3 * sizeof(double));
+            return ZS_OK;
+        }
         if (poses && P.K > 0) {
             ZS_CUDA(cudaMemcpy2DAsync(poses, 7 * sizeof(double), P.pose, kPoseStride * sizeof(double),
                                       7 * sizeof(double), P.K, cudaMemcpyDeviceToHost, h->stream));
@@ -1346,12 +1402,16 @@ int pose_only_solve(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_re
     const zs_ba_options& o = h->opt;
     const long long launches0 = launch_counter();
     const int cap = std::max(1, iterations * std::max(1, o.max_failures));
-    if (!h->po_out) ZS_CUDA(cudaMalloc(&h->po_out, sizeof(PoseOnlyOut)));
+    constexpr size_t kOut = (sizeof(PoseOnlyOut) + 15) / 16 * 16;  // the report, then the attempts
     if (h->po_hist_cap < cap) {
-        if (h->po_hist) ZS_CUDA(cudaFree(h->po_hist));
+        if (h->po_out) ZS_CUDA(cudaFree(h->po_out));
+        h->po_out = nullptr;
         h->po_hist = nullptr;
         h->po_hist_cap = 0;
-        ZS_CUDA(cudaMalloc(&h->po_hist, sizeof(zs_ba_attempt) * (size_t)cap));
+        char* buf = nullptr;
+        ZS_CUDA(cudaMalloc(&buf, kOut + sizeof(zs_ba_attempt) * (size_t)cap));
+        h->po_out = reinterpret_cast<PoseOnlyOut*>(buf);
+        h->po_hist = reinterpret_cast<zs_ba_attempt*>(buf + kOut);
         h->po_hist_cap = cap;
     }
     const size_t need = pose_only_scratch(h->P.M);
@@ -1368,11 +1428,17 @@ int pose_only_solve(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_re
     ZS_CUDA(launch_pose_only_lm(h->P, ctl, h->po_out, h->po_hist, h->po_scratch, s));
     ZS_CUDA(cudaEventRecord(h->ev1, s));
     PoseOnlyOut out{};
-    ZS_CUDA(cudaMemcpyAsync(&out, h->po_out, sizeof(out), cudaMemcpyDeviceToHost, s));
+    const size_t all = kOut + sizeof(zs_ba_attempt) * (size_t)cap;  // (cap bounds this solve's attempts)
+    char* stage = h->stage();
+    const size_t first = all <= kSmallCopy ? all : sizeof(out);
+    ZS_CUDA(cudaMemcpyAsync(stage, h->po_out, first, cudaMemcpyDeviceToHost, s));
     ZS_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&out, stage, sizeof(out));
     const int nh = std::min(out.history, h->po_hist_cap);
     h->history.assign((size_t)nh, zs_ba_attempt{});
-    if (nh > 0)
+    if (nh > 0 && first == all)
+        std::memcpy(h->history.data(), stage + kOut, sizeof(zs_ba_attempt) * (size_t)nh);
+    else if (nh > 0)
         ZS_CUDA(cudaMemcpy(h->history.data(), h->po_hist, sizeof(zs_ba_attempt) * (size_t)nh,
                            cudaMemcpyDeviceToHost));
     float ms = 0.f;
@@ -1495,15 +1561,27 @@ int zs_find_matches(zs_ba_handle* h, const uint8_t* lhs, int64_t lhs_count, cons
         uint8_t* dr = c.take<uint8_t>(32 * (size_t)nr);
         unsigned long long* part = c.take<unsigned long long>(chunks > 1 ? (size_t)chunks * nl * k : 1);
         unsigned long long* out = c.take<unsigned long long>((size_t)nl * k);
-        ZS_CUDA(cudaMemcpyAsync(dl, lhs, 32 * (size_t)nl, cudaMemcpyHostToDevice, h->stream));
-        if (nr > 0) ZS_CUDA(cudaMemcpyAsync(dr, rhs, 32 * (size_t)nr, cudaMemcpyHostToDevice, h->stream));
+        const size_t lb = 32 * (size_t)nl, rb = 32 * (size_t)nr, kb = sizeof(unsigned long long) * (size_t)nl * k;
+        char* stage = h->stage();
+        if (lb <= kSmallCopy && rb <= kSmallCopy) {  // (dr follows dl)
+            std::memcpy(stage, lhs, lb);
+            if (nr > 0) std::memcpy(stage + (dr - dl), rhs, rb);
+            ZS_CUDA(cudaMemcpyAsync(dl, stage, (size_t)(dr - dl) + rb, cudaMemcpyHostToDevice, h->stream));
+        } else {
+            ZS_CUDA(cudaMemcpyAsync(dl, lhs, lb, cudaMemcpyHostToDevice, h->stream));
+            if (nr > 0) ZS_CUDA(cudaMemcpyAsync(dr, rhs, rb, cudaMemcpyHostToDevice, h->stream));
+        }
         ZS_CUDA(cudaEventRecord(h->ev0, h->stream));
         launch_match(dl, nl, dr, nr, k, d_lim, chunks, part, out, h->stream);
         ZS_CUDA(cudaGetLastError());
         ZS_CUDA(cudaEventRecord(h->ev1, h->stream));
-        std::vector<unsigned long long> keys((size_t)nl * k);
-        ZS_CUDA(cudaMemcpyAsync(keys.data(), out, sizeof(unsigned long long) * keys.size(), cudaMemcpyDeviceToHost,
-                                h->stream));
+        // (the results' part of the staging buffer is not the descriptors')
+        char* results = stage + kStage / 2;
+        static_assert(2 * (kSmallCopy + 256) <= kStage / 2, "both fit");
+        const bool small = kb <= 2 * kSmallCopy;
+        std::vector<unsigned long long> big(small ? 0 : (size_t)nl * k);
+        const unsigned long long* keys = small ? reinterpret_cast<unsigned long long*>(results) : big.data();
+        ZS_CUDA(cudaMemcpyAsync(small ? (void*)results : (void*)big.data(), out, kb, cudaMemcpyDeviceToHost, h->stream));
         ZS_CUDA(cudaStreamSynchronize(h->stream));
         if (ms_device) {
             float ms = 0.f;
