@@ -1190,10 +1190,9 @@ void system_solve(zs_ba_handle* h) {
     DevProblem& P = h->P;
     DevWork& W = h->W;
     cudaStream_t s = h->stream;
-    launch_set_solve_ok(h->st, 1, s);
     {
         PhaseScope ps(h->timer, ZS_PHASE_INVERT, s);
-        launch_invert_w<T>(P, W, h->st, s);
+        launch_invert_w<T>(P, W, h->st, true, s);
     }
     {
         PhaseScope ps(h->timer, ZS_PHASE_SCHUR, s);
@@ -1238,8 +1237,7 @@ int solve_impl(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_report*
     linearize<T>(h);
     {
         PhaseScope ps(h->timer, ZS_PHASE_COST, s);
-        if (sizeof(T) == 4) launch_cost_fast(P, W, h->st, false, s);
-        else launch_cost(P, W, h->st, false, s);
+        launch_cost<T>(P, W, h->st, s);
         launch_init_lambda(P, W, h->st, o.tau, o.diagonal_clamp, s);
     }
     read_state(h);
@@ -1263,13 +1261,10 @@ int solve_impl(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_report*
             {
                 PhaseScope ps(h->timer, ZS_PHASE_UPDATE, s);
                 launch_update(P, W, h->st, s);
-                launch_scale(P, W, h->st, s);
             }
             {
                 PhaseScope ps(h->timer, ZS_PHASE_COST, s);
-                if (sizeof(T) == 4) launch_cost_fast(P, W, h->st, true, s);
-                else launch_cost(P, W, h->st, true, s);
-                launch_decide(h->st, s);
+                launch_decide<T>(P, W, h->st, s);
                 launch_rollback(P, h->st, s);
             }
             read_state(h);
@@ -1503,7 +1498,7 @@ int zs_ba_chi2(zs_ba_handle* h, double* chi2) {
             *chi2 = 0.0;
             return ZS_OK;
         }
-        launch_cost(h->P, h->W, h->st, false, h->stream);
+        launch_cost<double>(h->P, h->W, h->st, h->stream);
         read_state(h);
         *chi2 = h->st_host->chi2_new;
     } catch (const CudaError& e) {
@@ -1519,7 +1514,7 @@ int zs_ba_initial_lambda(zs_ba_handle* h, double* lambda) {
         ZS_CUDA(cudaSetDevice(h->device));
         if (h->tsize == 8) linearize<double>(h);
         else linearize<float>(h);
-        launch_cost(h->P, h->W, h->st, false, h->stream);
+        launch_cost<double>(h->P, h->W, h->st, h->stream);
         launch_init_lambda(h->P, h->W, h->st, h->opt.tau, h->opt.diagonal_clamp, h->stream);
         read_state(h);
         *lambda = h->st_host->lambda;
@@ -1795,7 +1790,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
             } else {
                 linearize<double>(h);
             }
-            launch_cost(P, W, h->st, false, s);
+            launch_cost<double>(P, W, h->st, s);
             launch_init_lambda(P, W, h->st, h->opt.tau, h->opt.diagonal_clamp, s);
             read_state(h);
             LmState init{};
@@ -1804,7 +1799,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
             init.solve_ok = 1;
             ZS_CUDA(cudaMemcpyAsync(h->st, &init, sizeof(LmState), cudaMemcpyHostToDevice, s));
             if (exact) launch_adj_check_lm(P, W, h->st, s);
-            launch_invert_w<double>(P, W, h->st, s);
+            launch_invert_w<double>(P, W, h->st, false, s);
             launch_schur<double>(P, W, h->st, s);
             ZS_CUDA(launch_chol_fx(n, W.S, (double*)W.F, W.fx, h->st, s));
             read_state(h);

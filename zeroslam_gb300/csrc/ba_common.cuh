@@ -127,6 +127,56 @@ __device__ inline void pose_plus(double* p, const double d[6]) {
     p[6] = nq[0];
 }
 
+// u0 v0 + u1 v1 with the first or the second product fused: which one is as
+// the compiler contracts the expressions of k_linearize and pose_plus, whose
+// results these are then bit for bit. (Under a robust loss the last bit of a
+// residual decides whether an outlier's weight gets its second-order term, so
+// that other roundings take other steps from the second one on.)
+__device__ __forceinline__ double dot2_first(double u0, double v0, double u1, double v1) {
+    return fma(u0, v0, __dmul_rn(u1, v1));
+}
+__device__ __forceinline__ double dot2_second(double u0, double v0, double u1, double v1) {
+    return fma(u1, v1, __dmul_rn(u0, v0));
+}
+
+// pose_plus in three parts that do not wait on one another, for three warps on
+// different SM quarters (its 230 FP64 instructions hold one quarter's pipe for
+// 15,000 cycles): the rotated quaternion, the rotated translation, the step's
+// left Jacobian; then joined.
+constexpr int kPlusParts = 16;
+__device__ inline void pose_plus_part(int part, const double* p, const double* d, double* out) {
+    if (part == 2) {
+        so3_left_jacobian(d, out + 7);
+        return;
+    }
+    double q[4];
+    so3_exp(d, q);
+    if (part == 0) {
+        const double r[4] = {p[6], p[3], p[4], p[5]};
+        out[0] = fma(-q[3], r[3], fma(-q[2], r[2], dot2_first(q[0], r[0], -q[1], r[1])));
+        out[1] = fma(-q[3], r[2], fma(q[2], r[3], dot2_first(q[0], r[1], q[1], r[0])));
+        out[2] = fma(q[3], r[1], fma(q[2], r[0], dot2_first(q[0], r[2], -q[1], r[3])));
+        out[3] = fma(q[3], r[0], fma(-q[2], r[1], dot2_first(q[0], r[3], q[1], r[2])));
+    } else {
+        const double t0 = fma(-q[3], p[2], fma(-q[2], p[1], -__dmul_rn(q[1], p[0])));
+        const double t1 = fma(-q[3], p[1], fma(q[2], p[2], __dmul_rn(q[0], p[0])));
+        const double t2 = fma(q[3], p[0], dot2_first(q[0], p[1], -q[1], p[2]));
+        const double t3 = fma(-q[2], p[0], dot2_first(q[0], p[2], q[1], p[1]));
+        out[4] = fma(t3, q[2], fma(-t2, q[3], dot2_second(t0, -q[1], t1, q[0])));
+        out[5] = fma(-t3, q[1], fma(t2, q[0], dot2_second(t0, -q[2], t1, q[3])));
+        out[6] = fma(t3, q[0], fma(t2, q[1], dot2_first(t0, -q[3], -t1, q[2])));
+    }
+}
+__device__ inline void pose_plus_join(const double* u, const double* d, double* p) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double dt = u[7 + 3 * i] * d[3] + u[8 + 3 * i] * d[4] + u[9 + 3 * i] * d[5];
+        p[i] = u[4 + i] + dt;
+        p[3 + i] = u[1 + i];
+    }
+    p[6] = u[0];
+}
+
 // Separately rounded IEEE operations (never fused into an FMA). The
 // residual and the squared error go through these so that every edge's
 // residual rounds exactly as the reference's double arithmetic does: the

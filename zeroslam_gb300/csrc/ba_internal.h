@@ -213,8 +213,9 @@ void launch_linearize(const DevProblem& P, DevWork& W, const int* go, cudaStream
 // kernel (or launch_adj_blocks) left: duplicates merged, H_ll, H_pp and b.
 template <typename T>
 void launch_block_sums(const DevProblem& P, DevWork& W, const int* go, cudaStream_t s);
+// begin: an attempt starts (st->solve_ok set, st->timeout cleared)
 template <typename T>
-void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
+void launch_invert_w(const DevProblem& P, DevWork& W, LmState* st, bool begin, cudaStream_t s);
 template <typename T>
 void launch_schur(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
 void launch_backsub(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
@@ -230,15 +231,15 @@ template <typename T>
 void launch_schur_pairs(const DevProblem& P, DevWork& W, const WinCtl* ctl, cudaStream_t s);
 void launch_update(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s);
 void launch_rollback(const DevProblem& P, const LmState* st, cudaStream_t s);
-void launch_scale(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s);
-// cost of the current state into st->chi2_new (when only_if_ok, skipped if !st->solve_ok)
-void launch_cost(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, cudaStream_t s);
-// the mixed form's cost (per-pose sandwich matrices of the current poses, then FP64 residuals)
-void launch_cost_fast(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, cudaStream_t s);
+// cost of the current state into st->chi2_new
+// (float: the mixed form's, per-pose sandwich matrices of the current poses, then FP64 residuals)
+template <typename T>
+void launch_cost(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s);
 void launch_pose_aux(const DevProblem& P, DevWork& W, cudaStream_t s);
 void launch_init_lambda(const DevProblem& P, DevWork& W, LmState* st, double tau, double clamp, cudaStream_t s);
-void launch_decide(LmState* st, cudaStream_t s);
-void launch_set_solve_ok(LmState* st, int v, cudaStream_t s);
+// the trial state's cost, the model's decrease and the decision
+template <typename T>
+void launch_decide(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s);
 
 // ---- batched windows (ba_batch.cu) ----
 constexpr int kBatchBuckets = 5;     // reduced-solve size buckets: n <= 64, 96, 128, 160, 192

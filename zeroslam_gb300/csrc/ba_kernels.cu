@@ -19,7 +19,7 @@
 //   k_backsub                                source/factor_graph.hpp:799-800
 //   k_update, k_rollback                     source/factor_graph.hpp:809-846, 947-960
 //   k_cost_partial                           get_current_chi    source/factor_graph.hpp:618-629
-//   k_scale_partial, k_decide                LM acceptance      source/factor_graph.hpp:555-606
+//   k_cost_partial, k_decide                 LM acceptance      source/factor_graph.hpp:555-606
 #include <algorithm>
 
 #include "ba_df.cuh"
@@ -132,12 +132,8 @@ __device__ __forceinline__ void plain_records(const double c0, const double c2, 
     for (int k = 0; k < 18; ++k) hrec[k] = 0.0;
 #pragma unroll
     for (int k = 0; k < kLmRec; ++k) lrec[k] = 0.0;
-    // u0 v0 + u1 v1 with the first or the second product fused, each as the
-    // compiler contracts the general code's expression: the results are that
-    // code's, bit for bit. (A landmark close to a camera's plane has entries
-    // that cancel to nothing in S, and another choice ends elsewhere.)
-    auto first = [](double u0, double v0, double u1, double v1) { return fma(u0, v0, __dmul_rn(u1, v1)); };
-    auto second = [](double u0, double v0, double u1, double v1) { return fma(u1, v1, __dmul_rn(u0, v0)); };
+    // (A landmark close to a camera's plane has entries that cancel to nothing
+    // in S, and another rounding ends elsewhere: dot2_first's comment.)
     if (!pf) {
         int k = 0;
 #pragma unroll
@@ -145,7 +141,7 @@ __device__ __forceinline__ void plain_records(const double c0, const double c2, 
 #pragma unroll
             for (int c = a; c < 6; ++c, ++k) {
                 const bool in0 = a != 4 && c != 4, in1 = a != 3 && c != 3;
-                if (in0 && in1) prec[k] = first(j0[a], j0[c], j1[a], j1[c]);
+                if (in0 && in1) prec[k] = dot2_first(j0[a], j0[c], j1[a], j1[c]);
                 else if (in0) prec[k] = j0[a] * j0[c];
                 else if (in1) prec[k] = j1[a] * j1[c];
             }
@@ -154,7 +150,7 @@ __device__ __forceinline__ void plain_records(const double c0, const double c2, 
         for (int a = 0; a < 6; ++a) {
             if (a == 3) prec[21 + a] = -(j0[a] * r[0]);
             else if (a == 4) prec[21 + a] = -(j1[a] * r[1]);
-            else prec[21 + a] = -second(j0[a], r[0], j1[a], r[1]);
+            else prec[21 + a] = -dot2_second(j0[a], r[0], j1[a], r[1]);
         }
         if (!lf) {
 #pragma unroll
@@ -163,19 +159,19 @@ __device__ __forceinline__ void plain_records(const double c0, const double c2, 
                 for (int c = 0; c < 3; ++c) {
                     if (a == 3) hrec[a * 3 + c] = j0[a] * l0[c];
                     else if (a == 4) hrec[a * 3 + c] = j1[a] * l1[c];
-                    else hrec[a * 3 + c] = second(j0[a], l0[c], j1[a], l1[c]);
+                    else hrec[a * 3 + c] = dot2_second(j0[a], l0[c], j1[a], l1[c]);
                 }
         }
     }
     if (!lf) {
-        lrec[0] = second(l0[0], l0[0], l1[0], l1[0]);
-        lrec[1] = second(l0[0], l0[1], l1[0], l1[1]);
-        lrec[2] = second(l0[0], l0[2], l1[0], l1[2]);
-        lrec[3] = second(l0[1], l0[1], l1[1], l1[1]);
-        lrec[4] = second(l0[1], l0[2], l1[1], l1[2]);
-        lrec[5] = second(l0[2], l0[2], l1[2], l1[2]);
+        lrec[0] = dot2_second(l0[0], l0[0], l1[0], l1[0]);
+        lrec[1] = dot2_second(l0[0], l0[1], l1[0], l1[1]);
+        lrec[2] = dot2_second(l0[0], l0[2], l1[0], l1[2]);
+        lrec[3] = dot2_second(l0[1], l0[1], l1[1], l1[1]);
+        lrec[4] = dot2_second(l0[1], l0[2], l1[1], l1[2]);
+        lrec[5] = dot2_second(l0[2], l0[2], l1[2], l1[2]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) lrec[6 + a] = -second(l0[a], r[0], l1[a], r[1]);
+        for (int a = 0; a < 3; ++a) lrec[6 + a] = -dot2_second(l0[a], r[0], l1[a], r[1]);
     }
 }
 
@@ -749,10 +745,14 @@ __global__ void __launch_bounds__(kThreads) k_reduce_pose_runs(DevProblem P, con
 }
 
 // Damped 3x3 landmark inverses (landmark_inverse); the plain form's row_exp is
-// cleared for k_w on the way.
+// cleared for k_w on the way, and with begin an attempt's flags are set.
 __global__ void __launch_bounds__(kThreads) k_invert(DevProblem P, const double* __restrict__ hll, double* hinv,
-                                                     float* hinv_f, int* lm_exp, int* row_exp, const LmState* st) {
+                                                     float* hinv_f, int* lm_exp, int* row_exp, LmState* st, int begin) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (begin && l == 0) {
+        st->solve_ok = 1;
+        st->timeout = 0;
+    }
     if (row_exp && l < 12 * P.K) row_exp[l] = kRowExpEmpty;
     if (l >= P.L) return;
     landmark_inverse(hll + (int64_t)l * 9, st->lambda, P.lm_fixed[l] != 0, hinv + (int64_t)l * 9,
@@ -1196,22 +1196,35 @@ __global__ void __launch_bounds__(kThreads) k_backsub(DevProblem P, const double
     delta[P.n + 3LL * l + lane] = I[0] * (bl[0] - u0) + I[1] * (bl[1] - u1) + I[2] * (bl[2] - u2);
 }
 
-// Backup and apply the step to free vertices.
+// Backup and apply the step to free vertices: blocks of 32 poses, three warps
+// a pose (pose_plus_part; one thread a pose took 12 us however few the poses,
+// this 8), then blocks of kThreads landmarks.
+constexpr int kUpdatePoses = 32;
 __global__ void __launch_bounds__(kThreads) k_update(DevProblem P, const double* __restrict__ delta, const LmState* st) {
+    __shared__ double parts[kUpdatePoses][kPlusParts + 1];
     if (!st->solve_ok) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < P.K) {
+    const int pose_blocks = (P.K + kUpdatePoses - 1) / kUpdatePoses;
+    if ((int)blockIdx.x < pose_blocks) {
+        const int i = threadIdx.x & 31, part = threadIdx.x >> 5, t = blockIdx.x * kUpdatePoses + i;
+        const bool mine = t < P.K && !P.pose_fixed[t];
         double* p = P.pose + (int64_t)t * kPoseStride;
-        double* bk = P.pose_bk + (int64_t)t * kPoseStride;
-#pragma unroll
-        for (int i = 0; i < kPoseStride; ++i) bk[i] = p[i];
-        if (P.pose_fixed[t]) return;
         double d[6];
+        if (mine && part < 3) {
 #pragma unroll
-        for (int i = 0; i < 6; ++i) d[i] = delta[6LL * t + i];
-        pose_plus(p, d);
-    } else if (t < P.K + P.L) {
-        const int l = t - P.K;
+            for (int m = 0; m < 6; ++m) d[m] = delta[6LL * t + m];
+            pose_plus_part(part, p, d, parts[i]);
+        }
+        if (part == 3 && t < P.K) {
+            double* bk = P.pose_bk + (int64_t)t * kPoseStride;
+#pragma unroll
+            for (int m = 0; m < kPoseStride; ++m) bk[m] = p[m];
+        }
+        __syncthreads();
+        if (mine && part == 0) pose_plus_join(parts[i], d, p);
+        return;
+    }
+    const int l = (blockIdx.x - pose_blocks) * blockDim.x + threadIdx.x;
+    if (l < P.L) {
         double* x = P.lm + (int64_t)l * kLmStride;
         double* bk = P.lm_bk + (int64_t)l * kLmStride;
 #pragma unroll
@@ -1242,79 +1255,70 @@ __global__ void __launch_bounds__(kThreads) k_rollback(DevProblem P, const LmSta
 
 // Fixed-shape two-level sums: kReduceBlocks blocks stride over the items in
 // a fixed order, then one block adds the block results in a fixed tree.
-__global__ void __launch_bounds__(kThreads) k_scale_partial(DevProblem P, const double* __restrict__ delta,
-                                                            const double* __restrict__ b, double* red,
-                                                            const LmState* st) {
-    __shared__ double sh[kThreads];
-    if (!st->solve_ok) return;
-    const double lam = st->lambda;
-    const int64_t N = (int64_t)P.n + 3LL * P.L;
-    double v = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        v += delta[i] * (lam * delta[i] + b[i]);
-    v = block_sum(v, sh);
-    if (threadIdx.x == 0) red[blockIdx.x] = v;
-}
+// The cost at the current state, the mixed form's (kFast) in FP64 through the
+// per-pose sandwich matrices (k_pose_aux of the current poses) with contracted
+// multiply-adds; of a trial also the model's decrease, by the same blocks
+// (blocks of their own took 72 us where the two take 54: the second half of
+// the grid is not spread over the SMs as the first is).
+struct Sum2 {
+    double a, b;
+    __device__ Sum2 operator+(const Sum2& o) const { return {a + o.a, b + o.b}; }
+};
 
-__global__ void __launch_bounds__(kThreads) k_cost_partial(DevProblem P, double* red, const LmState* st,
-                                                           int only_if_ok) {
-    __shared__ double sh[kThreads];
-    if (only_if_ok && !st->solve_ok) return;
-    double v = 0.0;
-    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < P.M; o += (int64_t)gridDim.x * blockDim.x) {
-        const int pi = P.obs_pose[o], li = P.obs_lm[o];
-        const double* pp = P.pose + (int64_t)pi * kPoseStride;
-        const double* xp = P.lm + (int64_t)li * kLmStride;
-        double p[7], X[3];
-#pragma unroll
-        for (int i = 0; i < 7; ++i) p[i] = pp[i];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) X[i] = xp[i];
+template <bool kFast>
+__global__ void __launch_bounds__(kThreads) k_cost_partial(DevProblem P, const double* __restrict__ aux,
+                                                           const double* __restrict__ delta,
+                                                           const double* __restrict__ b, double* red,
+                                                           const LmState* st, int trial) {
+    __shared__ Sum2 sh[kThreads];
+    if (trial && !st->solve_ok) return;
+    constexpr int64_t kStride = (int64_t)kReduceBlocks * kThreads;
+    const int64_t first = blockIdx.x * (int64_t)kThreads + threadIdx.x;
+    Sum2 v{0.0, 0.0};
+    for (int64_t o = first; o < P.M; o += kStride) {
+        const int pi = P.obs_pose[o];
+        const double* xp = P.lm + (int64_t)P.obs_lm[o] * kLmStride;
         const double2 uv = P.obs_uv[o];
-        double Xc[3], r[2];
-        residual(p, X, uv.x, uv.y, P.intr, Xc, r);
-        const double e2 = chi2_of(r, P.obs_info ? P.obs_info + 4 * o : nullptr);
-        if (P.loss.kind) {
-            double rho[3];
-            loss_rho(P.loss, e2, rho);
-            v += rho[0];
+        const double X[3] = {xp[0], xp[1], xp[2]};
+        const double* om = P.obs_info ? P.obs_info + 4 * o : nullptr;
+        if constexpr (kFast) {
+            v.a += cost_fast(aux + (int64_t)pi * kAux, X, uv.x, uv.y, P.intr, om, P.loss);
         } else {
-            v += e2;
+            const double* pp = P.pose + (int64_t)pi * kPoseStride;
+            double p[7];
+#pragma unroll
+            for (int i = 0; i < 7; ++i) p[i] = pp[i];
+            double Xc[3], r[2];
+            residual(p, X, uv.x, uv.y, P.intr, Xc, r);
+            const double e2 = chi2_of(r, om);
+            if (P.loss.kind) {
+                double rho[3];
+                loss_rho(P.loss, e2, rho);
+                v.a += rho[0];
+            } else {
+                v.a += e2;
+            }
         }
     }
-    v = block_sum(v, sh);
-    if (threadIdx.x == 0) red[blockIdx.x] = v;
-}
-
-// The mixed form's cost: FP64 through the per-pose sandwich matrices
-// (k_pose_aux of the current poses), contracted multiply-adds.
-__global__ void __launch_bounds__(kThreads) k_cost_partial_fast(DevProblem P, const double* __restrict__ aux,
-                                                                double* red, const LmState* st, int only_if_ok) {
-    __shared__ double sh[kThreads];
-    if (only_if_ok && !st->solve_ok) return;
-    double v = 0.0;
-    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < P.M; o += (int64_t)gridDim.x * blockDim.x) {
-        const double* xp = P.lm + (int64_t)P.obs_lm[o] * kLmStride;
-        const double X[3] = {xp[0], xp[1], xp[2]};
-        const double2 uv = P.obs_uv[o];
-        v += cost_fast(aux + (int64_t)P.obs_pose[o] * kAux, X, uv.x, uv.y, P.intr,
-                       P.obs_info ? P.obs_info + 4 * o : nullptr, P.loss);
+    if (trial) {
+        const double lam = st->lambda;
+        const int64_t N = (int64_t)P.n + 3LL * P.L;
+        for (int64_t i = first; i < N; i += kStride) v.b += delta[i] * (lam * delta[i] + b[i]);
     }
     v = block_sum(v, sh);
-    if (threadIdx.x == 0) red[blockIdx.x] = v;
+    if (threadIdx.x == 0) {
+        red[blockIdx.x] = v.a;
+        red[kReduceBlocks + blockIdx.x] = v.b;
+    }
 }
 
-// target: 0 = chi2_new, 1 = scale (+1e-3)
-__global__ void __launch_bounds__(kThreads) k_finish_sum(const double* red, LmState* st, int target, int only_if_ok) {
+// chi2_new from the cost's partials.
+__global__ void __launch_bounds__(kThreads) k_finish_cost(const double* red, LmState* st) {
     __shared__ double sh[kThreads];
-    if (only_if_ok && !st->solve_ok) return;
     double v = 0.0;
     for (int i = threadIdx.x; i < kReduceBlocks; i += kThreads) v += red[i];
     v = block_sum(v, sh);
-    if (threadIdx.x == 0) {
-        if (target == 0) st->chi2_new = v;
-        else st->scale = v + 1e-3;
-    }
+    if (threadIdx.x == 0) st->chi2_new = v;
 }
 
 __global__ void __launch_bounds__(kThreads) k_max_diag(DevProblem P, const double* __restrict__ hpp,
@@ -1340,20 +1344,40 @@ __global__ void __launch_bounds__(kThreads) k_max_diag(DevProblem P, const doubl
     if (threadIdx.x == 0) red[blockIdx.x] = sh[0];
 }
 
-__global__ void k_init_lambda(const double* red, LmState* st, double tau, double clamp) {
-    if (threadIdx.x != 0) return;
+__global__ void __launch_bounds__(kThreads) k_init_lambda(const double* red, LmState* st, double tau, double clamp) {
+    __shared__ double sh[kThreads];
     double m = 0.0;
-    for (int i = 0; i < kReduceBlocks; ++i) m = fmax(m, red[i]);
+    for (int i = threadIdx.x; i < kReduceBlocks; i += kThreads) m = fmax(m, red[i]);
+    sh[threadIdx.x] = m;
+    __syncthreads();
+    for (int s = kThreads / 2; s > 0; s >>= 1) {
+        if (threadIdx.x < s) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + s]);
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    m = sh[0];
     st->max_diag = m;
     st->lambda = tau * fmin(clamp, m);
     st->nu = 2.0;
     st->chi2 = st->chi2_new;
 }
 
-// source/factor_graph.hpp:542-591
-__global__ void k_decide(LmState* st) {
+// The trial's cost and the model's decrease (+1e-3) from their partials, and
+// the decision (source/factor_graph.hpp:542-591).
+__global__ void __launch_bounds__(kThreads) k_decide(const double* red, LmState* st) {
+    __shared__ Sum2 sh[kThreads];
+    const bool solved = st->solve_ok != 0;
+    if (solved) {
+        Sum2 v{0.0, 0.0};
+        for (int i = threadIdx.x; i < kReduceBlocks; i += kThreads) v = v + Sum2{red[i], red[kReduceBlocks + i]};
+        v = block_sum(v, sh);
+        if (threadIdx.x == 0) {
+            st->chi2_new = v.a;
+            st->scale = v.b + 1e-3;
+        }
+    }
     if (threadIdx.x != 0) return;
-    if (!st->solve_ok) {
+    if (!solved) {
         st->lambda *= st->nu;
         st->nu *= 2.0;
         st->good = 0;
@@ -1372,13 +1396,6 @@ __global__ void k_decide(LmState* st) {
         st->lambda *= st->nu;
         st->nu *= 2.0;
         st->good = 0;
-    }
-}
-
-__global__ void k_set_solve_ok(LmState* st, int v) {
-    if (threadIdx.x == 0) {
-        st->solve_ok = v;
-        st->timeout = 0;
     }
 }
 
@@ -1458,10 +1475,11 @@ void launch_w(const DevProblem& P, DevWork& W, cudaStream_t s) {
 }
 
 template <typename T>
-void launch_invert_w(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s) {
-    if (P.L > 0) {
+void launch_invert_w(const DevProblem& P, DevWork& W, LmState* st, bool begin, cudaStream_t s) {
+    if (P.L > 0 || begin) {
         k_invert<<<grid_for(std::max(P.L, W.row_exp ? 12 * P.K : 0)), kThreads, 0, s>>>(
-            P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, W.lm_exp, W.row_exp, st);
+            P, W.hll, W.hll_inv, sizeof(T) == 4 ? W.hll_inv_f : nullptr, W.lm_exp, W.row_exp, st,
+            begin ? 1 : 0);
         note_launch();
     }
     launch_w<T>(P, W, s);
@@ -1509,47 +1527,51 @@ void launch_backsub(const DevProblem& P, DevWork& W, const LmState* st, cudaStre
 }
 
 void launch_update(const DevProblem& P, DevWork& W, const LmState* st, cudaStream_t s) {
-    k_update<<<grid_for((int64_t)P.K + P.L), kThreads, 0, s>>>(P, W.delta, st); note_launch();
+    const int grid = (P.K + kUpdatePoses - 1) / kUpdatePoses + (P.L + kThreads - 1) / kThreads;
+    k_update<<<std::max(1, grid), kThreads, 0, s>>>(P, W.delta, st); note_launch();
 }
 
 void launch_rollback(const DevProblem& P, const LmState* st, cudaStream_t s) {
     k_rollback<<<grid_for((int64_t)P.K + P.L), kThreads, 0, s>>>(P, st); note_launch();
 }
 
-void launch_scale(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s) {
-    k_scale_partial<<<kReduceBlocks, kThreads, 0, s>>>(P, W.delta, W.b, W.red, st); note_launch();
-    k_finish_sum<<<1, kThreads, 0, s>>>(W.red, st, 1, 1); note_launch();
-}
-
-void launch_cost(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, cudaStream_t s) {
-    k_cost_partial<<<kReduceBlocks, kThreads, 0, s>>>(P, W.red, st, only_if_ok ? 1 : 0); note_launch();
-    k_finish_sum<<<1, kThreads, 0, s>>>(W.red, st, 0, only_if_ok ? 1 : 0); note_launch();
-}
-
 void launch_pose_aux(const DevProblem& P, DevWork& W, cudaStream_t s) {
     if (P.K > 0) { k_pose_aux<<<grid_for(P.K), kThreads, 0, s>>>(P, W.pose_aux, nullptr); note_launch(); }
 }
 
-void launch_cost_fast(const DevProblem& P, DevWork& W, LmState* st, bool only_if_ok, cudaStream_t s) {
-    launch_pose_aux(P, W, s);
-    k_cost_partial_fast<<<kReduceBlocks, kThreads, 0, s>>>(P, W.pose_aux, W.red, st, only_if_ok ? 1 : 0); note_launch();
-    k_finish_sum<<<1, kThreads, 0, s>>>(W.red, st, 0, only_if_ok ? 1 : 0); note_launch();
+template <typename T>
+static void launch_cost_partial(const DevProblem& P, DevWork& W, LmState* st, bool trial, cudaStream_t s) {
+    if (sizeof(T) == 4) launch_pose_aux(P, W, s);
+    k_cost_partial<sizeof(T) == 4><<<kReduceBlocks, kThreads, 0, s>>>(P, W.pose_aux, W.delta, W.b, W.red, st, trial);
+    note_launch();
+}
+
+template <typename T>
+void launch_cost(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s) {
+    launch_cost_partial<T>(P, W, st, false, s);
+    k_finish_cost<<<1, kThreads, 0, s>>>(W.red, st); note_launch();
+}
+
+template <typename T>
+void launch_decide(const DevProblem& P, DevWork& W, LmState* st, cudaStream_t s) {
+    launch_cost_partial<T>(P, W, st, true, s);
+    k_decide<<<1, kThreads, 0, s>>>(W.red, st); note_launch();
 }
 
 void launch_init_lambda(const DevProblem& P, DevWork& W, LmState* st, double tau, double clamp, cudaStream_t s) {
     k_max_diag<<<kReduceBlocks, kThreads, 0, s>>>(P, W.hpp, W.hll, W.red); note_launch();
-    k_init_lambda<<<1, 32, 0, s>>>(W.red, st, tau, clamp); note_launch();
+    k_init_lambda<<<1, kThreads, 0, s>>>(W.red, st, tau, clamp); note_launch();
 }
-
-void launch_decide(LmState* st, cudaStream_t s) { k_decide<<<1, 32, 0, s>>>(st); note_launch(); }
-
-void launch_set_solve_ok(LmState* st, int v, cudaStream_t s) { k_set_solve_ok<<<1, 32, 0, s>>>(st, v); note_launch(); }
 
 template void launch_linearize<double>(const DevProblem&, DevWork&, const int*, cudaStream_t);
 template void launch_linearize<float>(const DevProblem&, DevWork&, const int*, cudaStream_t);
 template void launch_block_sums<double>(const DevProblem&, DevWork&, const int*, cudaStream_t);
-template void launch_invert_w<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
-template void launch_invert_w<float>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
+template void launch_invert_w<double>(const DevProblem&, DevWork&, LmState*, bool, cudaStream_t);
+template void launch_cost<double>(const DevProblem&, DevWork&, LmState*, cudaStream_t);
+template void launch_decide<double>(const DevProblem&, DevWork&, LmState*, cudaStream_t);
+template void launch_invert_w<float>(const DevProblem&, DevWork&, LmState*, bool, cudaStream_t);
+template void launch_cost<float>(const DevProblem&, DevWork&, LmState*, cudaStream_t);
+template void launch_decide<float>(const DevProblem&, DevWork&, LmState*, cudaStream_t);
 template void launch_schur<double>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_schur<float>(const DevProblem&, DevWork&, const LmState*, cudaStream_t);
 template void launch_bs<double>(const DevProblem&, DevWork&, cudaStream_t);

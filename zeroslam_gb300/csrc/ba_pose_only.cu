@@ -69,18 +69,6 @@ __device__ __forceinline__ constexpr int place(int i, int j) {
     return i == 6 ? 21 + j : 6 * j - j * (j - 1) / 2 + (i - j);
 }
 
-// u0 v0 + u1 v1 with the first or the second product fused: which one is as
-// the compiler contracts the expressions of k_linearize and pose_plus, whose
-// results these are then bit for bit. (Under a robust loss the last bit of a
-// residual decides whether an outlier's weight gets its second-order term, so
-// that other roundings take other steps from the second one on.)
-__device__ __forceinline__ double first(double u0, double v0, double u1, double v1) {
-    return fma(u0, v0, __dmul_rn(u1, v1));
-}
-__device__ __forceinline__ double second(double u0, double v0, double u1, double v1) {
-    return fma(u1, v1, __dmul_rn(u0, v0));
-}
-
 struct Observed {
     double X[3], Xc[3], r[2];
     const double* om;
@@ -129,8 +117,8 @@ __device__ __forceinline__ void add_terms(const DevProblem& P, const double p[7]
     if (om) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) W[i] = om[i];
-        orr0 = first(om[0], r[0], om[1], r[1]);
-        orr1 = first(om[2], r[0], om[3], r[1]);
+        orr0 = dot2_first(om[0], r[0], om[1], r[1]);
+        orr1 = dot2_first(om[2], r[0], om[3], r[1]);
     }
     if (P.loss.kind) {
         const double e2 = chi2_of(r, om);
@@ -164,20 +152,20 @@ __device__ __forceinline__ void add_terms(const DevProblem& P, const double p[7]
             A0 = j1[a] * W[2];
             A1 = j1[a] * W[3];
         } else {
-            A0 = second(j0[a], W[0], j1[a], W[2]);
-            A1 = second(j0[a], W[1], j1[a], W[3]);
+            A0 = dot2_second(j0[a], W[0], j1[a], W[2]);
+            A1 = dot2_second(j0[a], W[1], j1[a], W[3]);
         }
 #pragma unroll
         for (int c = a; c < 6; ++c) {
             double& t = acc[place(c, a)];
             if (c == 3) t += __dmul_rn(A0, j0[c]);
             else if (c == 4) t += __dmul_rn(A1, j1[c]);
-            else t += first(A0, j0[c], A1, j1[c]);
+            else t += dot2_first(A0, j0[c], A1, j1[c]);
         }
         double& t = acc[21 + a];
         if (a == 3) t -= __dmul_rn(j0[a], g0);
         else if (a == 4) t -= __dmul_rn(j1[a], g1);
-        else t -= second(j0[a], g0, j1[a], g1);
+        else t -= dot2_second(j0[a], g0, j1[a], g1);
     }
 }
 
@@ -223,7 +211,7 @@ struct Shared {
     double sys[2][MF][kSys];
     double delta[MF][6];
     double lo[MF], hi[MF];  // of a pose's L_ii; lo = 0 where a pivot failed
-    double plus[MF][16];    // a trial pose's parts: quaternion, rotated translation, the step's left Jacobian
+    double plus[MF][kPlusParts];  // a trial pose's parts (pose_plus_part)
     double gain[64];        // the poses' shares of the model's gain
     double red[NT];
     double wpart[NT / 32][kRec];
@@ -303,32 +291,7 @@ template <int MK, int MF, int NT>
 __device__ void trial_state(int b, Shared<MK, MF, NT>& sh) {
     static_assert(NT >= 128 && MF <= 32 && MK <= 64, "a warp per part, a lane per free pose");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nf = sh.nfree;
-    if (warp < 3 && lane < nf) {
-        const double* p = sh.pose[b][sh.order[lane]];
-        const double* d = sh.delta[lane];
-        double* out = sh.plus[lane];
-        if (warp == 2) {
-            so3_left_jacobian(d, out + 7);
-        } else {
-            double q[4];
-            so3_exp(d, q);
-            if (warp == 0) {
-                const double r[4] = {p[6], p[3], p[4], p[5]};
-                out[0] = fma(-q[3], r[3], fma(-q[2], r[2], first(q[0], r[0], -q[1], r[1])));
-                out[1] = fma(-q[3], r[2], fma(q[2], r[3], first(q[0], r[1], q[1], r[0])));
-                out[2] = fma(q[3], r[1], fma(q[2], r[0], first(q[0], r[2], -q[1], r[3])));
-                out[3] = fma(q[3], r[0], fma(-q[2], r[1], first(q[0], r[3], q[1], r[2])));
-            } else {
-                const double t0 = fma(-q[3], p[2], fma(-q[2], p[1], -__dmul_rn(q[1], p[0])));
-                const double t1 = fma(-q[3], p[1], fma(q[2], p[2], __dmul_rn(q[0], p[0])));
-                const double t2 = fma(q[3], p[0], first(q[0], p[1], -q[1], p[2]));
-                const double t3 = fma(-q[2], p[0], first(q[0], p[2], q[1], p[1]));
-                out[4] = fma(t3, q[2], fma(-t2, q[3], second(t0, -q[1], t1, q[0])));
-                out[5] = fma(-t3, q[1], fma(t2, q[0], second(t0, -q[2], t1, q[3])));
-                out[6] = fma(t3, q[0], fma(t2, q[1], second(t0, -q[3], -t1, q[2])));
-            }
-        }
-    }
+    if (warp < 3 && lane < nf) pose_plus_part(warp, sh.pose[b][sh.order[lane]], sh.delta[lane], sh.plus[lane]);
     if (warp == 3) {
         if (lane < nf) {
             double sc = 0.0;
@@ -345,16 +308,7 @@ __device__ void trial_state(int b, Shared<MK, MF, NT>& sh) {
     }
     __syncthreads();
     if (threadIdx.x < nf) {
-        double* t = sh.pose[b ^ 1][sh.order[threadIdx.x]];
-        const double* u = sh.plus[threadIdx.x];
-        const double* d = sh.delta[threadIdx.x];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double dt = u[7 + 3 * i] * d[3] + u[8 + 3 * i] * d[4] + u[9 + 3 * i] * d[5];
-            t[i] = u[4 + i] + dt;
-            t[3 + i] = u[1 + i];
-        }
-        t[6] = u[0];
+        pose_plus_join(sh.plus[threadIdx.x], sh.delta[threadIdx.x], sh.pose[b ^ 1][sh.order[threadIdx.x]]);
     }
     __syncthreads();
 }
