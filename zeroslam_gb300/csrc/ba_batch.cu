@@ -101,39 +101,54 @@ __global__ void __launch_bounds__(kThreads) k_bs_init(DevProblem P, const double
     S[P.win_s_off[w] + idx] = v;
 }
 
-// delta_l = H_ll^-1 (b_l - H_lp delta_p), as k_backsub.
+// delta_l = H_ll^-1 (b_l - H_lp delta_p), as k_backsub: eight lanes a landmark.
+// Mixed form: delta_p in FP32 (delta_f) and its products widened on the integer
+// pipe, which leaves 3 of 12 FP64 instructions an observation; the gathers of
+// the records bound it then (214 -> 201 us at 256 windows, 6.5 million
+// observations; the FP64 form, which had a thread a landmark as well, 105 -> 99
+// at 64 windows).
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_bbacksub(DevProblem P, const T* __restrict__ hpl,
                                                        const double* __restrict__ hinv, const double* __restrict__ b,
-                                                       double* delta, const LmState* __restrict__ st,
-                                                       const WinCtl* __restrict__ ctl) {
-    constexpr int RS = sizeof(T) == 4 ? 20 : 18;
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= P.L) return;
-    const int w = P.lm_win[l];
-    if (!ctl[w].active || !st[w].solve_ok) return;
-    const double* bl = b + P.n + 3LL * l;
-    double v0 = bl[0], v1 = bl[1], v2 = bl[2];
-    const int e = P.lm_ptr[l + 1];
-    for (int o = P.lm_ptr[l]; o < e; ++o) {
+                                                       double* delta, const float* __restrict__ delta_f,
+                                                       const LmState* __restrict__ st, const WinCtl* __restrict__ ctl) {
+    constexpr int RS = sizeof(T) == 4 ? 20 : 18, kLanes = 8;
+    const int lane = threadIdx.x & (kLanes - 1);
+    const int64_t l = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kLanes;
+    bool in = l < P.L;  // (every lane stays for the butterfly)
+    if (in) {
+        const int w = P.lm_win[l];
+        in = ctl[w].active && st[w].solve_ok;
+    }
+    double u0 = 0.0, u1 = 0.0, u2 = 0.0;
+    const int e = in ? P.lm_ptr[l + 1] : 0;
+    for (int o = in ? P.lm_ptr[l] + lane : 0; o < e; o += kLanes) {
         if (!P.blk_valid[o]) continue;
         const T* h = hpl + (int64_t)P.pm[o] * RS;
-        const double* dp = delta + 6LL * P.obs_pose[o];
+        const int64_t p = 6LL * P.obs_pose[o];
         T s0 = T(0), s1 = T(0), s2 = T(0);
 #pragma unroll
         for (int a = 0; a < 6; ++a) {
-            const T d = (T)dp[a];
+            T d;
+            if constexpr (sizeof(T) == 4) d = delta_f[p + a];
+            else d = delta[p + a];
             s0 += h[a * 3] * d;
             s1 += h[a * 3 + 1] * d;
             s2 += h[a * 3 + 2] * d;
         }
-        v0 -= s0; v1 -= s1; v2 -= s2;
+        u0 += widen(s0); u1 += widen(s1); u2 += widen(s2);
     }
-    const double* I = hinv + (int64_t)l * 9;
-    double* dl = delta + P.n + 3LL * l;
-    dl[0] = I[0] * v0 + I[1] * v1 + I[2] * v2;
-    dl[1] = I[3] * v0 + I[4] * v1 + I[5] * v2;
-    dl[2] = I[6] * v0 + I[7] * v1 + I[8] * v2;
+    __syncwarp();
+#pragma unroll
+    for (int off = kLanes / 2; off > 0; off >>= 1) {
+        u0 += __shfl_xor_sync(0xffffffffu, u0, off);
+        u1 += __shfl_xor_sync(0xffffffffu, u1, off);
+        u2 += __shfl_xor_sync(0xffffffffu, u2, off);
+    }
+    if (lane >= 3 || !in) return;
+    const double* bl = b + P.n + 3LL * l;
+    const double* I = hinv + (int64_t)l * 9 + 3 * lane;
+    delta[P.n + 3LL * l + lane] = I[0] * (bl[0] - u0) + I[1] * (bl[1] - u1) + I[2] * (bl[2] - u2);
 }
 
 // Backup and apply the step to the free vertices of windows whose solve passed.
@@ -591,7 +606,10 @@ __global__ void k_bsolve(BatchView V, const int32_t* __restrict__ list, int coun
                 }
             }
             mark(3);
-            for (int i = tid; i < n; i += blockDim.x) V.delta[6LL * p0 + i] = xs[i];
+            for (int i = tid; i < n; i += blockDim.x) {
+                V.delta[6LL * p0 + i] = xs[i];
+                if (V.delta_f) V.delta_f[6LL * p0 + i] = (float)xs[i];
+            }
         }
         if (V.prof && tid == 0) V.prof[(int64_t)w * kBatchProfSlots + 4] += sweeps;
         if (tid == 0) {
@@ -691,7 +709,9 @@ cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, con
         const cudaError_t e = launch_chol_fx_windows(*B.fx, P.nwin, W.S, B.st, B.ctl, s);
         if (e != cudaSuccess) return e;
     }
-    BatchView V{W.S, W.bs, W.delta, B.st, B.ctl, P.win_pose0, P.win_s_off, B.prof};
+    // (the mixed form's FP32 copy of delta_p: pose_aux is free until the update has moved the poses)
+    float* delta_f = sizeof(T) == 4 ? reinterpret_cast<float*>(W.pose_aux) : nullptr;
+    BatchView V{W.S, W.bs, W.delta, delta_f, B.st, B.ctl, P.win_pose0, P.win_s_off, B.prof};
     const int refine = sizeof(T) == 4 ? prm.refine_iters : 0;
     cudaError_t e = cudaEventRecord(B.ev_fork, s);
     if (e != cudaSuccess) return e;
@@ -707,7 +727,8 @@ cudaError_t launch_batch_round(const DevProblem& P, DevWork& W, BatchDev& B, con
         if ((e = cudaStreamWaitEvent(s, B.ev_join[b], 0)) != cudaSuccess) return e;
     }
     if (P.L > 0) {
-        k_bbacksub<T><<<grid_for(P.L), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.b, W.delta, B.st, B.ctl);
+        k_bbacksub<T><<<grid_for(8LL * P.L), kThreads, 0, s>>>(P, (const T*)W.hpl, W.hll_inv, W.b, W.delta, delta_f, B.st,
+                                                               B.ctl);
         note_launch();
     }
     k_bupdate<<<grid_for((int64_t)P.K + P.L), kThreads, 0, s>>>(P, W.delta, B.st, B.ctl); note_launch();
@@ -785,7 +806,7 @@ cudaError_t bsolve_autotune(int bucket, int sms, cudaStream_t s, int* threads_ou
     if (err == cudaSuccess) {
         k_tune_fill<<<grid_for(nn * nwin), kThreads, 0, s>>>(n, nwin, S, bs, st, ctl, pose0, soff, list);
         chk(cudaGetLastError());
-        BatchView V{S, bs, delta, st, ctl, pose0, soff, nullptr};
+        BatchView V{S, bs, delta, nullptr, st, ctl, pose0, soff, nullptr};
         const int cand[5] = {64, 128, 256, 512, 1024};
         for (int c = 0; c < 5 && err == cudaSuccess; ++c) {
             const int t = cand[c];

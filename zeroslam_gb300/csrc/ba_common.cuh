@@ -177,6 +177,16 @@ __device__ inline void pose_plus_join(const double* u, const double* d, double* 
     p[6] = u[0];
 }
 
+__device__ __forceinline__ double widen(double v) { return v; }
+// (double)f on the integer pipe: a conversion holds the FP64 pipe as long as a
+// multiply-add does. Subnormals, infinities and NaN are converted as usual.
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), m = u << 1;
+    if (m == 0) return __hiloint2double((int)u, 0);
+    if (m < 0x01000000u || m >= 0xff000000u) return (double)f;
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
 // Separately rounded IEEE operations (never fused into an FMA). The
 // residual and the squared error go through these so that every edge's
 // residual rounds exactly as the reference's double arithmetic does: the

@@ -272,6 +272,7 @@ struct BatchView {
     double* S;
     const double* bs;
     double* delta;
+    float* delta_f;  // mixed form: delta_p in FP32, else null
     LmState* st;
     WinCtl* ctl;
     const int32_t* win_pose0;
