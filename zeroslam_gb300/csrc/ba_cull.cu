@@ -18,7 +18,9 @@
 // L2. The terms are FP64 with the reference's rounding order and no
 // contraction (the _rn intrinsics), so the means, and with them the
 // decisions, are the reference's bit for bit. The kernel is bound by the
-// FP64 pipe (a division and a square root per observation), not by memory.
+// FP64 pipe (some 36 instructions' time an observation, a division's among
+// them), not by memory: square roots, conversions and additions of zero off
+// that pipe took the kernel from 89 us to 79 at 773,087 observations.
 //
 // k_pose_rt gives the frames of the solver's resident poses: the rotation
 // matrix and translation that map::optimise writes back into each frame
@@ -36,6 +38,39 @@ constexpr int kCullRecent = 7;          // source/map.hpp:282
 constexpr float kCullError = 5.991f;    // source/map.hpp:304,316
 constexpr double kMinDepth = 1.0e-12;   // source/camera.hpp:98
 
+// The float nearest to the double nearest to sqrt(v), on the integer pipe (the
+// FP64 square root and the conversion hold the FP64 pipe as long as ten
+// multiply-adds). v = a 2^e, e even, 2^52 <= a < 2^54: the float is 8 q 2^(e /
+// 2), q the integer nearest to sqrt(a) / 8, from FP32's square root of a's
+// upper half and exact comparisons of a with the squares of the midpoints 8 q
+// +- 4. Within a few units of such a square, where the rounding to double
+// decides, and outside the ranges the two roundings are made as they stand.
+__device__ __forceinline__ float sqrt_to_float(double v) {
+    const long long bits = __double_as_longlong(v);
+    const int ex = (int)(bits >> 52);  // (a sign makes it negative)
+    if (ex > 1023 - 100 && ex < 1023 + 200) {
+        int e = ex - 1023 - 52;
+        long long a = (bits & ((1ll << 52) - 1)) | (1ll << 52);
+        if (e & 1) {
+            a <<= 1;
+            --e;
+        }
+        long long q = (long long)(int)(sqrtf((float)(unsigned)(a >> 22)) * 256.f);
+        long long d = a - 64 * q * q;  // a - (8 q)^2
+        while (d >= 64 * q + 16) {
+            d -= 64 * (2 * q + 1);
+            ++q;
+        }
+        while (d <= 16 - 64 * q) {
+            d += 64 * (2 * q - 1);
+            --q;
+        }
+        if (d < 64 * q + 8 && d > 24 - 64 * q)
+            return (float)(int)q * __int_as_float(((e >> 1) + 3 + 127) << 23);
+    }
+    return __double2float_rn(__dsqrt_rn(v));
+}
+
 // One observation's term: the landmark mapped into the frame, R X + t with
 // the row sums of source/matrix.hpp:494-509 (starting from 0), projected as
 // camera.hpp:97-111, and the distance of matrix.hpp:177-183 rounded to float.
@@ -44,8 +79,8 @@ __device__ __forceinline__ float cull_term(const double* __restrict__ Rt, const 
     double m[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        double s = 0.0;
-        s = __dadd_rn(s, __dmul_rn(__ldg(Rt + 3 * i + 0), X0));
+        // (without the reference's addition to 0, which changes no value)
+        double s = __dmul_rn(__ldg(Rt + 3 * i + 0), X0);
         s = __dadd_rn(s, __dmul_rn(__ldg(Rt + 3 * i + 1), X1));
         s = __dadd_rn(s, __dmul_rn(__ldg(Rt + 3 * i + 2), X2));
         m[i] = __dadd_rn(s, __ldg(Rt + 9 + i));
@@ -56,14 +91,11 @@ __device__ __forceinline__ float cull_term(const double* __restrict__ Rt, const 
     const double py = __dadd_rn(__dmul_rn(__ldg(in + 1), __dmul_rn(m[1], iz)), __ldg(in + 3));
     const double dx = __dsub_rn(kx, px);
     const double dy = __dsub_rn(ky, py);
-    double ls = 0.0;
-    ls = __dadd_rn(ls, __dmul_rn(dx, dx));
-    ls = __dadd_rn(ls, __dmul_rn(dy, dy));
-    return __double2float_rn(__dsqrt_rn(ls));
+    return sqrt_to_float(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
 }
 
-__device__ __forceinline__ double kp_x(const float2& k) { return (double)k.x; }
-__device__ __forceinline__ double kp_y(const float2& k) { return (double)k.y; }
+__device__ __forceinline__ double kp_x(const float2& k) { return widen(k.x); }
+__device__ __forceinline__ double kp_y(const float2& k) { return widen(k.y); }
 __device__ __forceinline__ double kp_x(const double2& k) { return k.x; }
 __device__ __forceinline__ double kp_y(const double2& k) { return k.y; }
 
