@@ -268,6 +268,8 @@ int zs_ba_get_history(zs_ba_handle* h, zs_ba_attempt* out, int32_t capacity, int
  * Gauss-Newton part.
  * With a = the gradient vector b of zs_ba_linear_step, v is the exact Newton
  * step. FP64 handles and ZS_LOSS_NONE only (ZS_ERR_UNSUPPORTED otherwise).
+ * ZS_ERR_CHOLESKY (neither matrix can be factored) and ZS_ERR_TIMEOUT (a
+ * bounded device wait ran out) leave the outputs as they were.
  * No counterpart in the reference. */
 int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dloss_dlandmark, double* dloss_duv,
                   double* dloss_dintrinsics, double* adjoint_state, zs_ba_adjoint_report* rep);

@@ -1844,8 +1844,14 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
             int it = 0;
             const int max_it = 200;
             if (anorm > 0.0) {
+                // (the triangular solve's waits are bounded: its state is read
+                // at every wait of the host)
+                auto copy_state = [&] {
+                    ZS_CUDA(cudaMemcpyAsync(h->st_host, h->st, sizeof(LmState), cudaMemcpyDeviceToHost, s));
+                };
                 precondition(r, z);
                 launch_adj_copy(N, z, pv, s);
+                copy_state();
                 double rz = dot(r, z);
                 if (h->opt.verbose)
                     std::fprintf(stderr, "zs adjoint: |a| %.6e  r.Mr %.6e  |M^-1 a| %.6e\n", anorm, rz,
@@ -1865,7 +1871,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 double* red2 = W.red + kReduceBlocks;  // the loop's partial sums
                 AdjCg ch = c0;
                 const int batch = exact ? 2 : 8;
-                while (!ch.done) {
+                while (h->st_host->solve_ok && !ch.done) {
                     for (int b = 0; b < batch; ++b) {
                         launch_adj_residual(P, h->adj_rec, pv, zero, h->adj_part, W.opch_sum, q, s);  // q = -H p
                         launch_adj_dot(N, pv, q, red2, s);
@@ -1880,6 +1886,7 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                         launch_adj_cg_axpby(N, cg, 1, z, pv, s);       // p = z + beta p
                     }
                     ZS_CUDA(cudaMemcpyAsync(&ch, cg, sizeof(AdjCg), cudaMemcpyDeviceToHost, s));
+                    copy_state();
                     ZS_CUDA(cudaStreamSynchronize(s));
                     if (h->opt.verbose)
                         std::fprintf(stderr, "zs adjoint: it %3d  |r|/|a| %.6e  done %d\n", ch.it, ch.rn / anorm,
@@ -1889,6 +1896,10 @@ int zs_ba_adjoint(zs_ba_handle* h, const double* dloss_dpose, const double* dlos
                 // the true residual of the returned v
                 launch_adj_residual(P, h->adj_rec, v, a, h->adj_part, W.opch_sum, r, s);
                 rn = std::sqrt(dot(r, r));
+            }
+            if (!h->st_host->solve_ok) {  // a solve gave up on the way: v is no solution
+                status = h->st_host->timeout ? ZS_ERR_TIMEOUT : ZS_ERR_CHOLESKY;
+                dloss_duv = dloss_dintrinsics = adjoint_state = nullptr;
             }
             // outputs from v
             double* duv_dev = h->adj_part;  // 2M doubles of scratch
