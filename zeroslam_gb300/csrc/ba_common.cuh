@@ -295,7 +295,9 @@ __device__ inline double cost_fast(const double* __restrict__ a, const double* _
 // ignores the failed inversion (source/factor_graph.hpp:763). of (optional,
 // mixed form) also receives the inverse in FP32, padded to 12 floats; oe
 // (optional, plain form) s, about half the exponent of the inverse's largest
-// entry: H_pl 2^s and H_pl H_ll^-1 2^-s are then of like size.
+// entry: H_pl 2^s and H_pl H_ll^-1 2^-s are then of like size; kLmExpNone for
+// a zero inverse.
+constexpr int kLmExpNone = 1 << 20;
 __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double lam, bool fixed, double* o,
                                         float* of, int* oe) {
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -327,7 +329,10 @@ __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double
     if (oe) {
         const double m = fmax(fabs(v[0]), fmax(fabs(v[4]), fabs(v[8])));
         const int e = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
-        *oe = e == 0 || e == 0x7ff ? 0 : (e - 1022) >> 1;
+        long long any = 0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) any |= __double_as_longlong(v[i]) << 1;
+        *oe = any == 0 ? kLmExpNone : e == 0 || e == 0x7ff ? 0 : (e - 1022) >> 1;
     }
     if (of) {
         float4* f = reinterpret_cast<float4*>(of);

@@ -763,7 +763,9 @@ __global__ void __launch_bounds__(kThreads) k_invert(DevProblem P, const double*
 // floats per landmark) and 16-byte record loads and stores. Plain form: also
 // the exponents of each pose row's largest entries (row_exp, cleared before),
 // of H_pl 2^s and of W 2^-s, s = lm_exp of the landmark: the scales of the
-// fixed-point records.
+// fixed-point records. (A landmark without an inverse has no part in the
+// products and none in the scales: an H_pl that nothing balances may be any
+// number of bits above the others.)
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_w(DevProblem P, const T* __restrict__ hpl, const double* __restrict__ hinv,
                                                 const float* __restrict__ hinv_f, T* __restrict__ W,
@@ -805,8 +807,8 @@ __global__ void __launch_bounds__(kThreads) k_w(DevProblem P, const T* __restric
                     mw = max(mw, fixed::exponent(w[a * 3 + c]));
                 }
                 // (values that are not finite stay recognisable)
-                eh[a] = mh > 1024 ? 8192 : mh + s;
-                ew[a] = mw > 1024 ? 8192 : mw - s;
+                eh[a] = mh > 1024 ? 8192 : s == kLmExpNone ? kRowExpEmpty : mh + s;
+                ew[a] = mw > 1024 ? 8192 : s == kLmExpNone ? kRowExpEmpty : mw - s;
             }
 #pragma unroll
             for (int i = 0; i < 9; ++i) w2[i] = make_double2(w[2 * i], w[2 * i + 1]);
@@ -928,7 +930,8 @@ constexpr int kSchurFrac = 58;
 constexpr int kSchurMinExp = -990;  // rows below 2^-990 (or all zero) are scaled by that: the scales stay normal
 
 // H_pl 2^s and W 2^-s of one observation in fixed point, 10 x 16 bytes each:
-// rows 0-2 and rows 3-5 of the 6 x 3 block, 9 pairs and a pad.
+// rows 0-2 and rows 3-5 of the 6 x 3 block, 9 pairs and a pad; zeros where the
+// landmark has no inverse.
 __global__ void __launch_bounds__(kThreads) k_schur_fix(DevProblem P, const double* __restrict__ W,
                                                         const double* __restrict__ hpl, const int* __restrict__ lm_exp,
                                                         const int* __restrict__ row_exp, int4* __restrict__ fxw,
@@ -939,6 +942,11 @@ __global__ void __launch_bounds__(kThreads) k_schur_fix(DevProblem P, const doub
     const int64_t o = P.pose_obs[q];
     if (!P.blk_valid[o]) return;
     const int s = lm_exp[P.obs_lm[o]];
+    if (s == kLmExpNone) {
+#pragma unroll
+        for (int i = 0; i < 10; ++i) fxh[q * 10 + i] = fxw[q * 10 + i] = make_int4(0, 0, 0, 0);
+        return;
+    }
     int bad = 0;
     auto convert = [&](const double* src, const int* e, int sign, int4* dst) {
         const double2* v2 = reinterpret_cast<const double2*>(src);
