@@ -42,3 +42,18 @@ def test_neighbours_keep_their_bits(zs_lib, depth):
             if (i, j) != (pose, pose):
                 assert np.array_equal(SA[i, :, j], SB[i, :, j]), (i, j)
 
+
+
+@pytest.mark.parametrize("depth,lam", [(3.0, 1e-6), (3.0, 1e-2), (0.3, 1e-4), (0.3, 1.0), (1e-2, 1e-2), (1e-2, 100.0)])
+def test_damping_alone_holds_it(zs_lib, oracle, depth, lam):
+    """The same landmark where the damping makes its block regular: the inverse
+    is up to 10^12 times larger along the ray, along which H_pl has no part."""
+    sc = scenes.arc_scene(6, 90, seed=61)
+    pose, K = 2, sc.K
+    two = _with_near(sc, pose, depth)
+    a, b = _step(sc, lam), _step(two, lam)
+    d = np.sqrt(lam + np.concatenate([np.diag(h) for h in oracle.linear_step(two, lam)["hpp"].reshape(K, 6, 6)]))
+    err = np.tril(np.abs(a["S"] - b["S"])) / (d[:, None] * d[None, :])
+    err[6 * pose:6 * pose + 6, 6 * pose:6 * pose + 6] = 0.0
+    # a pair's sum of at most L products, each rounded at 2^-53 of the two rows' own scale
+    assert err.max() <= two.L * 2.0**-53

@@ -289,15 +289,34 @@ constexpr int kPoseAux = 24;
 __device__ inline double cost_fast(const double* __restrict__ a, const double* __restrict__ X, double u_obs,
                                    double v_obs, const Intrinsics& in, const double* om, const LossParams& loss);
 
+constexpr int kLmExpNone = 1 << 20;
+
+// For H_pl = J_p^T J_l and V = H_ll + lambda I = sum J_l^T J_l + lambda I: J_l is
+// of size sqrt(m), m V's largest diagonal entry, and J_l V^-1 of size g = max over
+// H_ll's eigenvalues u of sqrt(u) / (u + lambda): 1 / sqrt(m) for the large ones, and
+// for the smallest, u + lambda = 1 / w (w the inverse's largest diagonal entry),
+// sqrt(u) w. Both sides are J_p's size times the same factor with 2^s =
+// sqrt(g / sqrt(m)). Along a direction that only the damping holds (a landmark
+// seen once) u is 0 and H_pl has no part, however large the inverse is there:
+// balanced by w alone, H_pl stood up to 2^20 above the other records of its rows
+// (u below m 2^-46 counts as 0: it is rounding by then).
+__device__ inline int landmark_balance(const double m, const double w, double lam) {
+    auto exponent = [](double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1022; };
+    const int em = exponent(m), ew = exponent(w);
+    if (em == -1022 || em == 1025 || ew == -1022 || ew == 1025) return 0;  // none, not finite, subnormal
+    const double u = 1.0 / w - lam;
+    int g2 = -em;  // of g^2
+    if (u > 0.0 && exponent(u) > em - 46) g2 = max(g2, exponent(u) + 2 * ew);
+    return (g2 - em + 2) >> 2;
+}
+
 // matrix::invert<3> of H_ll + lambda I for one landmark
 // (source/matrix.hpp:749-774): fixed landmarks and singular blocks
 // (|det| <= 1e-12 max|a|^3) get a zero inverse, as solve_linear_system
 // ignores the failed inversion (source/factor_graph.hpp:763). of (optional,
 // mixed form) also receives the inverse in FP32, padded to 12 floats; oe
-// (optional, plain form) s, about half the exponent of the inverse's largest
-// entry: H_pl 2^s and H_pl H_ll^-1 2^-s are then of like size; kLmExpNone for
-// a zero inverse.
-constexpr int kLmExpNone = 1 << 20;
+// (optional, plain form) the exponent s that makes H_pl 2^s and H_pl H_ll^-1
+// 2^-s alike (landmark_balance); kLmExpNone for a zero inverse.
 __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double lam, bool fixed, double* o,
                                         float* of, int* oe) {
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -327,12 +346,12 @@ __device__ inline void landmark_inverse(const double* __restrict__ hll_l, double
 #pragma unroll
     for (int i = 0; i < 9; ++i) o[i] = v[i];
     if (oe) {
-        const double m = fmax(fabs(v[0]), fmax(fabs(v[4]), fabs(v[8])));
-        const int e = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
         long long any = 0;
 #pragma unroll
         for (int i = 0; i < 9; ++i) any |= __double_as_longlong(v[i]) << 1;
-        *oe = any == 0 ? kLmExpNone : e == 0 || e == 0x7ff ? 0 : (e - 1022) >> 1;
+        const double w = fmax(fabs(v[0]), fmax(fabs(v[4]), fabs(v[8])));
+        const double m = fmax(fabs(hll_l[0]), fmax(fabs(hll_l[4]), fabs(hll_l[8]))) + lam;
+        *oe = any == 0 ? kLmExpNone : landmark_balance(m, w, lam);
     }
     if (of) {
         float4* f = reinterpret_cast<float4*>(of);
