@@ -155,13 +155,15 @@ __global__ void __launch_bounds__(kThreads) k_adj_blocks(DevProblem P, const dou
     for (int i = 6; i < 12; ++i) lh[i] = 0.0;
 }
 
+// The blocks as they stand: a direction that only the damping (1e-13 of the
+// largest diagonal entry) would hold is left to the Gauss-Newton
+// preconditioner and its 10^4 times larger one.
 __global__ void __launch_bounds__(kThreads) k_adj_check_lm(DevProblem P, const double* __restrict__ hll, LmState* st) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= P.L || P.lm_fixed[l]) return;
     double a[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) a[i] = hll[(int64_t)l * 9 + i];
-    a[0] += st->lambda; a[4] += st->lambda; a[8] += st->lambda;
     const double d2 = a[0] * a[4] - a[1] * a[3];
     const double det = a[0] * (a[4] * a[8] - a[7] * a[5]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);
     const double m = fmax(a[0], fmax(a[4], a[8]));

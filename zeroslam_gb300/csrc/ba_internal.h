@@ -321,8 +321,8 @@ void launch_adj_prep(const DevProblem& P, double* rec, cudaStream_t s);
 // The exact Hessian's blocks per observation, from the records, where
 // launch_linearize leaves the Gauss-Newton ones.
 void launch_adj_blocks(const DevProblem& P, const double* rec, DevWork& W, cudaStream_t s);
-// st->solve_ok = 0 unless every free landmark's H_ll + lambda I is positive
-// definite and passes the inverse's determinant test.
+// st->solve_ok = 0 unless every free landmark's H_ll is positive definite and
+// passes the inverse's determinant test.
 void launch_adj_check_lm(const DevProblem& P, const DevWork& W, LmState* st, cudaStream_t s);
 void launch_adj_residual(const DevProblem& P, const double* rec, const double* v, const double* a, double* part,
                          double* csum, double* out, cudaStream_t s);
