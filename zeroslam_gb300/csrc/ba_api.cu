@@ -33,8 +33,13 @@ namespace {
 // Triples per Schur segment (a warp's share): 512, or in FP64 fewer where the
 // problem has too few of them to give every SM quarter four warps (152 x 4 x
 // 4), but at least four rounds of the warp's eight triples. The mixed form
-// keeps 512: its FP32 sums depend on the split.
+// keeps 512: its FP32 sums depend on the split. So do an FP64 sum's last bits,
+// and a window's must not depend on the windows beside it: in a batch every
+// segment has 128 (64 / 128 / 256 / 512 took 38.6 / 36.9 / 36.4 / 36.5 ms for 64
+// windows of up to 30 poses and 3,000 landmarks, ten iterations, and 2.85 / 2.92 /
+// 3.04 / 3.12 for 8 of up to 8 and 400).
 constexpr int64_t kSegment = 512;
+constexpr int64_t kSegmentBatch = 128;
 constexpr int64_t kSegmentMin = 32;
 constexpr int64_t kSchurWarps = 152 * 16;
 
@@ -907,7 +912,9 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
     pair_i.reserve(npairs);
     pair_j.reserve(npairs);
     const int64_t seg_len =
-        h->tsize == 4 ? kSegment : std::clamp((ntriples / kSchurWarps + 7) / 8 * 8, kSegmentMin, kSegment);
+        h->tsize == 4 ? kSegment
+        : batched     ? kSegmentBatch
+                      : std::clamp((ntriples / kSchurWarps + 7) / 8 * 8, kSegmentMin, kSegment);
     for (int w = 0; w < nwin; ++w) {
         const int64_t kw = wp[w + 1] - wp[w];
         for (int64_t k = key_base[w]; k < key_base[w + 1]; ++k) {
