@@ -1023,15 +1023,23 @@ static void build_problem(zs_ba_handle* h, const zs_ba_problem* p, const std::ve
         W.jac = dalloc<ObsJac>((size_t)M, own);
         W.jp_pm = dalloc<float4>(3 * (size_t)M, own);
         W.hll_inv_f = dalloc<float>(12 * (size_t)std::max(L, 1), own);
+        W.pose_part = dalloc<char>(ts * 28 * M, own);  // record-major, 27 values padded to 28
     }
     else {
-        W.lm_part = dalloc<char>(ts * 12 * M, own);  // record-major, 9 values padded to 12
-        W.fxw = dalloc<int4>(10 * (size_t)M, own);
-        W.fxh = dalloc<int4>(10 * (size_t)M, own);
+        // The linearisation's records (record-major, 9 values padded to 12 and 27
+        // to 28), which are summed right after it, and the Schur products' in
+        // fixed point, which each attempt forms anew, share 320 bytes an observation.
+        auto bytes = [&](size_t record) { return (record * (size_t)M + 255) / 256 * 256; };
+        constexpr size_t kLmRec = 12 * sizeof(double), kPoseRec = 28 * sizeof(double), kFxRec = 10 * sizeof(int4);
+        static_assert(kLmRec + kPoseRec == 2 * kFxRec, "the same size");
+        char* rec = dalloc<char>(std::max(bytes(kLmRec) + bytes(kPoseRec), 2 * bytes(kFxRec)), own);
+        W.lm_part = rec;
+        W.pose_part = rec + bytes(kLmRec);
+        W.fxw = reinterpret_cast<int4*>(rec);
+        W.fxh = reinterpret_cast<int4*>(rec + bytes(kFxRec));
         W.row_exp = dalloc<int>(12 * (size_t)K, own);
         W.lm_exp = dalloc<int>((size_t)std::max(L, 1), own);
     }
-    W.pose_part = dalloc<char>(ts * 28 * M, own);  // record-major, 27 values padded to 28
     W.hpp = dalloc<double>((size_t)K * 36, own);
     W.hll = dalloc<double>((size_t)L * 9, own);
     W.hll_inv = dalloc<double>((size_t)L * 9, own);

@@ -129,8 +129,8 @@ struct DevWork {
     void* W = nullptr;         // [M*RS] T, pose-major positions
     double* pose_aux = nullptr; // [K*24] mixed form: per-pose sandwich matrix, translation, rotation
     double* partial = nullptr; // [nsegs*36] Schur segment sums (FP64)
-    int4* fxw = nullptr;       // plain form: [M*10] W in fixed point, pose-major positions
-    int4* fxh = nullptr;       // plain form: [M*10] H_pl in fixed point
+    int4* fxw = nullptr;       // plain form: [M*10] W in fixed point, pose-major positions (with fxh in the
+    int4* fxh = nullptr;       // plain form: [M*10] H_pl in fixed point (memory of lm_part and pose_part)
     int* row_exp = nullptr;    // plain form: [12K] exponents of the scales of each pose's rows: H_pl (6K), W (6K)
     int* lm_exp = nullptr;     // plain form: [L] exponents of the landmarks' balance
     void* lm_part = nullptr;   // plain form: [M*12] per-observation landmark records (9 used)
