@@ -487,7 +487,8 @@ __device__ bool accumulate(const Fx& d, int i, int j, Smem<T>& sm, Acc<T / 16, T
 }
 
 __device__ __forceinline__ ll load_scaled(const Fx& d, int row, int col, int& bad) {
-    const double v = row < d.n && col < d.n ? __ldg(d.S + (int64_t)row * d.n + col) : (row == col ? 1.0 : 0.0);
+    // (not by the read-only path: the windows' factors are written over S in the same launch)
+    const double v = row < d.n && col < d.n ? d.S[(int64_t)row * d.n + col] : (row == col ? 1.0 : 0.0);
     return quantize(v, kFrac - d.e[row] - d.e[col], bad);
 }
 
