@@ -224,7 +224,9 @@ int zs_ba_set_batch(zs_ba_handle* h, int num_windows, const zs_ba_problem* windo
 /* Solves every window of the batch as zs_ba_solve would (same iterations /
  * use_relative semantics per window). window_reports (may be NULL): one
  * report per window; rep (may be NULL): the batch summary. Returns the
- * accepted steps summed over windows, or a negative status. A batch whose
+ * accepted steps summed over windows, or a negative status (ZS_ERR_TIMEOUT: a
+ * bounded device wait of a window's factor ran out; that window's report has it
+ * too and it stops at its last accepted state, the others are solved). A batch whose
  * landmarks are all fixed (tracking problems) takes the pose-only path
  * (options.pose_only_path): one launch, one CTA per window, in FP64. */
 int zs_ba_solve_batch(zs_ba_handle* h, int iterations, int use_relative, zs_ba_report* window_reports,
@@ -432,7 +434,9 @@ int zs_ba_cull(zs_ba_handle* h, const int32_t* landmark_id, const int32_t* pose_
  * row-major n x n matrix A = L L^T and solves L L^T x = b. L (n*n, lower, zero
  * above the diagonal) and x may be NULL. precision: ZS_PRECISION_FP64, or
  * ZS_PRECISION_MIXED (the mixed solve's preconditioner: FP32 factor and its
- * inverse, then FP64 refinement of x).
+ * inverse, then FP64 refinement of x). FP64 sums in fixed point: the errors of
+ * L and x are FP64's or less against the scale of their row, sqrt(A_ii), but
+ * entries below 2^-60 of it are lost.
  * Returns ZS_OK, ZS_ERR_CHOLESKY, ZS_ERR_TIMEOUT (a bounded wait between
  * the factor's tile tasks ran out; nothing hangs) or a CUDA status. */
 int zs_dense_cholesky_solve(const double* A, int n, const double* b, double* L, double* x, int precision);

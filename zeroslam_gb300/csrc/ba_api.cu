@@ -1285,7 +1285,7 @@ int solve_impl(zs_ba_handle* h, int iterations, bool use_relative, zs_ba_report*
             read_state(h);
             r.attempts++;
             if (hs.timeout) {  // a bounded device wait ran out: the solve stops with the state restored
-                std::snprintf(g_last_error, sizeof(g_last_error), "a dependency wait of the preconditioner ran out");
+                std::snprintf(g_last_error, sizeof(g_last_error), "a dependency wait of the reduced system's factor or solve ran out");
                 r.status = ZS_ERR_TIMEOUT;
                 if (rep) *rep = r;
                 return ZS_ERR_TIMEOUT;

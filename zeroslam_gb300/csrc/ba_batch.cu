@@ -447,7 +447,7 @@ __global__ void k_bsolve(BatchView V, const int32_t* __restrict__ list, int coun
     double* sc = bv + NMAX;                            // [NMAX] Jacobi scale (mixed form), else 1
     TF* dinv = reinterpret_cast<TF*>(sc + NMAX);       // [NMAX] 1 / L_ii
     TF* vt = dinv + NMAX;                              // [NMAX] solve vector in TF
-    TF* eps = vt + NMAX;                               // [NMAX] per-row pivot threshold
+    TF* eps = vt + NMAX;                               // [NMAX] per-row pivot threshold (the mixed form's factor)
     TF* A = eps + NMAX;                                // tiles
     __shared__ int s_idx, s_flag;
     __shared__ double s_red[32];

@@ -501,9 +501,12 @@ cudaError_t launch_preconditioner(int n, const double* S, float* F, float* X, fl
 // launch runs the whole LM loop (FP64) on the poses in P.pose. Device memory:
 // out, hist (hist_cap attempt records), scratch (pose_only_scratch(M) doubles).
 constexpr int kPoseOnlyMaxK = 64;
-// At most this many free poses: each free pose's sums take one pass of the
-// grid (the FP64 pipe bounds it), so problems with more free poses are
-// faster on the general path (measured: 16 free poses 2.42 against 2.03 ms).
+// At most this many free poses; problems with more take the general path. The
+// line was drawn for a kernel that took a pass of the grid for each free pose.
+// The present one takes one pass for all and, built with room for 32, was faster
+// at every count: 5 / 8 / 16 / 32 free poses in 201 / 227 / 378 / 705 us against
+// 944 / 1069 / 1212 / 1700 (1,500 landmarks) and 434 / 571 / 987 / 1854 against
+// 1538 / 1358 / 1650 / 2352 (6,000).
 constexpr int kPoseOnlyMaxFree = 4;
 struct PoseOnlyCtl {
     double tau, clamp, legacy_stop, rel_tol, floor;
